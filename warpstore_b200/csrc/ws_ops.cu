@@ -54,247 +54,294 @@ struct RowTemplate {
   u64 w[kMaxRowWords];
 };
 namespace {
-__global__ void kFillRows(u64* rows, int64_t nrows, int rw, RowTemplate t, int64_t emptyRows) {
-  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < nrows; i += (int64_t)gridDim.x * blockDim.x) {
-    u64* r = rows + i * rw;
-    for (int j = 1; j < rw; ++j) r[j] = t.w[j];
-    r[0] = i < emptyRows ? kEmpty : 0ull;
-  }
-}
-
-// Exclusive scan of n counts in place (one CTA); counts[n] receives the total.
-__global__ void kScanExclusive(int64_t* counts, int64_t n) {
-  __shared__ int64_t part[1024];
-  const int t = threadIdx.x, T = blockDim.x;
-  const int64_t per = (n + T - 1) / T;
-  const int64_t lo = min((int64_t)t * per, n), hi = min(lo + per, n);
-  int64_t s = 0;
-  for (int64_t i = lo; i < hi; ++i) s += counts[i];
-  part[t] = s;
-  __syncthreads();
-  for (int off = 1; off < T; off <<= 1) {  // Hillis-Steele inclusive scan of the thread sums
-    const int64_t v = t >= off ? part[t - off] : 0;
-    __syncthreads();
-    part[t] += v;
-    __syncthreads();
-  }
-  int64_t run = t ? part[t - 1] : 0;
-  for (int64_t i = lo; i < hi; ++i) {
-    const int64_t c = counts[i];
-    counts[i] = run;
-    run += c;
-  }
-  if (t == T - 1) counts[n] = part[T - 1];
-}
-
-// Occupied result rows: hash rows [0, cap) by their key word, the extra row (cap) by its claim flag,
-// dense rows by slot 0 (COUNT(*)) being non-zero.
-struct OccSpec {
-  int rw, mode;  // mode 1 dense, 2 hash
-  int cnt0;      // word of slot 0
-  int64_t cap;   // hash: index of the extra row
+// Result rows to their identities (hash rows empty: key word kEmpty, the extra row's claim flag 0) and the
+// control words to 0.
+struct FillSpec {
+  u64* rows;
+  int64_t words;       // rows x rw
+  int64_t emptyWords;  // hash rows x rw: their word 0 is kEmpty, every other row's 0
+  int rw;
+  u64* ctl;            // kCtlWords words
+  RowTemplate t;
 };
-__device__ __forceinline__ bool occupied(const u64* rows, int64_t i, const OccSpec& s) {
-  const u64* r = rows + i * s.rw;
+constexpr int kCtlWords = 4;
+// Thread `tid` of `nthreads` (at least rw).  The threads step by a multiple of the row width, so each stays
+// on one word of the rows (a constant) and a warp's stores are consecutive: 2^24 rows of 32 B take 79 us,
+// against 310 us with a row per thread (and 345 us with a loop of its own for the key words).
+__device__ __forceinline__ void fillRows(const FillSpec& f, int64_t tid, int64_t nthreads) {
+  if (tid < kCtlWords) f.ctl[tid] = 0;
+  const int64_t step = nthreads / f.rw * f.rw;
+  if (tid >= step) return;
+  const int j = (int)(tid % f.rw);
+  const u64 v = j == 0 ? kEmpty : f.t.w[j];
+  const int64_t plain = j == 0 ? f.emptyWords : f.words;  // one loop for every lane: whole sectors per store
+  for (int64_t i = tid; i < f.words; i += step) f.rows[i] = i < plain ? v : 0ull;
+}
+__global__ void kFillRows(const __grid_constant__ FillSpec f) {
+  fillRows(f, blockIdx.x * (int64_t)blockDim.x + threadIdx.x, (int64_t)gridDim.x * blockDim.x);
+}
+__global__ void kFillRowsMany(const FillSpec* fs) {  // spec blockIdx.y
+  fillRows(fs[blockIdx.y], blockIdx.x * (int64_t)blockDim.x + threadIdx.x, (int64_t)gridDim.x * blockDim.x);
+}
+
+// ---- result delivery.  Occupied result rows (hash rows [0, cap) by their key word, the extra row (cap) by
+// its claim flag, dense rows by slot 0 (COUNT(*)) being non-zero) become groups in ascending row order:
+// keys in the engine's format, accs in its slot format, exact words.
+//
+// A result table of at most kSmallRows rows is delivered by one CTA in one launch (kDeliver: occupancy,
+// ranks, groups and the status), whole queries' worth of them by one launch of a CTA each (kDeliverMany); a
+// larger one by two (kOccCount, whose last CTA also scans the chunks' counts; kEmitChunks).  The separate
+// count, scan, status, index, emit and convert launches they replace cost a small query 13 to 25 us of
+// launches and each read the table again.  The groups' row indices are listed in shared memory and the
+// output is written by consecutive words, so that stores to pinned host memory go out as whole lines.
+struct ResultSpec {
+  const u64* rows;
+  int64_t nrows, cap;  // cap: index of the extra hash row
+  const int* err;
+  const double* tkeys;
+  int rw, mode;        // mode 0 no keys, 1 dense, 2 hash
+  int cnt0;            // word of slot 0
+  int nk, na;
+  uint8_t kind[WS_MAX_AGGS];     // kind of the slot whose words the slot shows (its partner's for SK_NONE)
+  uint8_t derived[WS_MAX_AGGS];  // SK_NONE: the high half of a split BIGINT SUM
+  uint8_t aggBits[WS_MAX_AGGS], aggPart[WS_MAX_AGGS];
+  int16_t woff[WS_MAX_AGGS];
+  uint8_t keyInt[WS_MAX_KEYS];
+  int64_t kmin[WS_MAX_KEYS], range[WS_MAX_KEYS], stride[WS_MAX_KEYS];
+};
+// Where groups [first, first + limit) go (null: not wanted): row-major from output row 0, or column-major
+// in columns of colRows.
+struct OutSpec {
+  double* keys;
+  double* accs;
+  long long* exact;
+  int64_t first, limit, colRows;
+};
+constexpr int64_t kSmallRows = 4097;
+constexpr int kDeliverThreads = 1024, kDeliverIters = (int)((kSmallRows + kDeliverThreads - 1) / kDeliverThreads);
+constexpr int kOccChunk = 2048, kOccThreads = 256;
+
+__device__ __forceinline__ bool occupied(const ResultSpec& s, int64_t i) {
+  const u64* r = s.rows + i * s.rw;
   if (s.mode == 0) return true;  // no GROUP BY: the one result row
   if (s.mode == 1) return r[s.cnt0] != 0;
   if (i == s.cap) return r[0] != 0;
   return r[0] != kEmpty;
 }
-constexpr int kOccChunk = 2048;
-__global__ void kOccCount(const u64* rows, int64_t nrows, OccSpec s, int64_t* counts) {
-  __shared__ int wc[32];
-  const int64_t c0 = (int64_t)blockIdx.x * kOccChunk;
-  int c = 0;
-  for (int64_t i = c0 + threadIdx.x; i < min(c0 + kOccChunk, nrows); i += blockDim.x) c += occupied(rows, i, s);
-  for (int o = 16; o > 0; o >>= 1) c += __shfl_down_sync(0xffffffffu, c, o);
-  if ((threadIdx.x & 31) == 0) wc[threadIdx.x >> 5] = c;
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    int t = 0;
-    for (int w = 0; w < (int)(blockDim.x >> 5); ++w) t += wc[w];
-    counts[blockIdx.x] = t;
+__device__ __forceinline__ double keyOut(const ResultSpec& s, int64_t i, int k) {
+  if (s.mode == 1) {
+    const long long v = s.kmin[k] + (i / s.stride[k]) % s.range[k];
+    return s.keyInt[k] ? __longlong_as_double(v) : (double)v;
   }
+  if (s.nk == 1 && i != s.cap) return __longlong_as_double((long long)s.rows[i * s.rw]);
+  return s.tkeys[i * s.nk + k];
 }
-__global__ void kOccWrite(const u64* rows, int64_t nrows, OccSpec s, const int64_t* offs, int64_t* idx) {
-  __shared__ int wbase[32];
-  __shared__ int64_t run;
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
-  const int64_t c0 = (int64_t)blockIdx.x * kOccChunk;
-  if (threadIdx.x == 0) run = offs[blockIdx.x];
-  __syncthreads();
-  for (int64_t b = c0; b < min(c0 + kOccChunk, nrows); b += blockDim.x) {
-    const int64_t i = b + threadIdx.x;
-    const bool occ = i < nrows && i < c0 + kOccChunk && occupied(rows, i, s);
-    const unsigned m = __ballot_sync(0xffffffffu, occ);
-    if (lane == 0) wbase[warp] = __popc(m);
-    __syncthreads();
-    int before = 0, total = 0;
-    for (int w = 0; w < nw; ++w) {
-      if (w < warp) before += wbase[w];
-      total += wbase[w];
-    }
-    if (occ) idx[run + before + __popc(m & ((1u << lane) - 1))] = i;
-    __syncthreads();
-    if (threadIdx.x == 0) run += total;
-    __syncthreads();
-  }
+// Exact words of slot a of result row i: (lo, hi) of an integer SUM, (value, 0) otherwise.
+__device__ __forceinline__ void exactOut(const ResultSpec& s, int64_t i, int a, long long& w0, long long& w1) {
+  const u64* r = s.rows + i * s.rw + s.woff[a];
+  const uint8_t k = s.kind[a];
+  w0 = (long long)r[0];
+  w1 = k == SK_ISUM ? (long long)r[1] : 0;
+  if (k == SK_DMIN || k == SK_DMAX) w0 = __double_as_longlong(dunord(w0));
 }
-
-// Result rows -> keys (engine format) and exact words per group.
-struct EmitSpec {
-  int nk, na, rw, mode;  // mode 0 no keys, 1 dense, 2 hash
-  uint8_t kind[WS_MAX_AGGS];
-  int16_t woff[WS_MAX_AGGS];
-  int16_t partner[WS_MAX_AGGS];
-  uint8_t keyInt[WS_MAX_KEYS];
-  int64_t kmin[WS_MAX_KEYS], range[WS_MAX_KEYS], stride[WS_MAX_KEYS];
-  const double* tkeys;
-  int64_t cap;
-};
-// Keys (engine format) and exact words of result row i: key k at kout[k * kstride], slot a at
-// xout[2a], xout[2a + 1].
-__device__ __forceinline__ void emitRow(const u64* rows, int64_t i, const EmitSpec& s, double* kout, int64_t kstride,
-                                        long long* xout) {
-  const u64* r = rows + i * s.rw;
-  for (int k = 0; k < s.nk; ++k) {
-    double kv;
-    if (s.mode == 1) {
-      const long long v = s.kmin[k] + (i / s.stride[k]) % s.range[k];
-      kv = s.keyInt[k] ? __longlong_as_double(v) : (double)v;
-    } else if (s.nk == 1 && i != s.cap) {
-      kv = __longlong_as_double((long long)r[0]);
-    } else {
-      kv = s.tkeys[i * s.nk + k];
-    }
-    kout[k * kstride] = kv;
-  }
-  for (int a = 0; a < s.na; ++a) {
-    const int src = s.kind[a] == SK_NONE ? s.partner[a] : a;
-    const int o = s.woff[src];
-    long long w0 = (long long)r[o], w1 = 0;
-    const uint8_t k = s.kind[src];
-    if (k == SK_ISUM) w1 = (long long)r[o + 1];
-    else if (k == SK_DMIN || k == SK_DMAX) w0 = __double_as_longlong(dunord(w0));
-    xout[2 * a] = w0;
-    xout[2 * a + 1] = w1;
-  }
-}
-
-__global__ void kEmit(const u64* rows, const int64_t* idx, int64_t m, EmitSpec s, double* keys, int64_t* exact,
-                      int colMajor) {
-  for (int64_t j = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; j < m; j += (int64_t)gridDim.x * blockDim.x) {
-    const int64_t i = idx ? idx[j] : j;
-    emitRow(rows, i, s, colMajor ? keys + j : keys + j * s.nk, colMajor ? m : 1, (long long*)exact + j * s.na * 2);
-  }
-}
-
-// Fetch straight into host memory (pinned and mapped): group p (ascending result-row order; the groups
-// of chunk b of kOccChunk result rows are offs[b]..) goes to output row p - first when first <= p <
-// first + limit.  One sub-tile of blockDim result rows at a time, its rows staged in shared memory
-// ([blockDim][nk + 2 na] words) and stored as contiguous words (whole PCIe writes rather than one
-// 8-byte write per word of a row).  Nothing is written when the run raised a flag (hash overflow, dense
-// key out of range, staged-copy timeout): the caller reads the status and reruns.
-__global__ void kOccEmitHost(const u64* rows, int64_t nrows, OccSpec o, EmitSpec s, const int64_t* offs, int64_t nchunks,
-                             const int* err, int64_t first, int64_t limit, double* keys, long long* exact) {
-  extern __shared__ long long stg[];
-  __shared__ int wbase[32];
-  if (err[0] || err[2] || (o.mode == 2 && err[1])) return;
-  if (offs[blockIdx.x + 1] <= first || offs[blockIdx.x] >= first + limit) return;  // none of this chunk's groups
-  const int64_t last = first + limit;
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
-  const int xw = 2 * s.na, rw = s.nk + xw;
-  const int64_t c0 = (int64_t)blockIdx.x * kOccChunk, cend = min(c0 + kOccChunk, nrows);
-  int64_t run = offs[blockIdx.x];
-  for (int64_t b = c0; b < cend; b += blockDim.x) {
-    const int64_t i = b + threadIdx.x;
-    const bool occ = i < cend && occupied(rows, i, o);
-    const unsigned m = __ballot_sync(0xffffffffu, occ);
-    if (lane == 0) wbase[warp] = __popc(m);
-    __syncthreads();
-    int before = 0, total = 0;
-    for (int w = 0; w < nw; ++w) {
-      if (w < warp) before += wbase[w];
-      total += wbase[w];
-    }
-    if (occ) {
-      long long* r = stg + (int64_t)(before + __popc(m & ((1u << lane) - 1))) * rw;
-      emitRow(rows, i, s, (double*)r, 1, r + s.nk);
-    }
-    __syncthreads();
-    // this sub-tile's groups [run, run + total) clipped to [first, last), at output row p - first
-    const int lo = (int)min((int64_t)total, max((int64_t)0, first - run));
-    const int hi = (int)max((int64_t)lo, min((int64_t)total, last - run));
-    for (int t = lo * s.nk + threadIdx.x; t < hi * s.nk; t += blockDim.x)
-      keys[(run - first) * s.nk + t] = __longlong_as_double(stg[(t / s.nk) * rw + t % s.nk]);
-    for (int t = lo * xw + threadIdx.x; t < hi * xw; t += blockDim.x)
-      exact[(run - first) * xw + t] = stg[(t / xw) * rw + s.nk + t % xw];
-    run += total;
-    __syncthreads();
-  }
-}
-
-// Status of an asynchronous fetch, in host memory (pinned and mapped).
-__global__ void kFetchStatus(const int64_t* total, const int* err, int hashMode, ws_fetch_status* st) {
-  st->groups = *total;
-  st->overflow = hashMode && err[1] ? 1 : 0;
-  st->error = err[0] ? WS_ERR_RANGE : err[2] ? WS_ERR_INTERNAL : 0;
-}
-
-// Exact words -> the engine's double slot format, on the device (for compact()).
-struct DblSpec {
-  int na, nokeys;
-  uint8_t kind[WS_MAX_AGGS], aggBits[WS_MAX_AGGS], aggPart[WS_MAX_AGGS];
-};
-__device__ __host__ inline double bitsToD(long long v) {
-  double d;
-  memcpy(&d, &v, 8);
-  return d;
-}
-__device__ __host__ inline double slotDouble(const DblSpec& s, int a, long long w0, long long w1, bool srcIsNone,
-                                             uint8_t srcKind) {
-  const uint8_t k = srcKind;
+// The engine's double slot format of those words.
+__device__ __forceinline__ double accOut(const ResultSpec& s, int a, long long w0, long long w1) {
+  const uint8_t k = s.kind[a];
   if (k == SK_COUNT) return (double)w0;
   if (k == SK_ISUM) {
     const __int128 T = (__int128)(((unsigned __int128)(unsigned long long)w1 << 64) | (unsigned long long)w0);
-    if (s.nokeys) {
-      long long lo = w0;
-      double d;
-      memcpy(&d, &lo, 8);
-      return d;
-    }
-    if (s.aggBits[a]) {
-      long long v = s.aggPart[a] == 2 || srcIsNone ? (long long)(T >> 32) : s.aggPart[a] == 1 ? (long long)(T & 0xffffffff) : w0;
-      double d;
-      memcpy(&d, &v, 8);
-      return d;
-    }
+    if (s.nk == 0) return __longlong_as_double(w0);
+    if (s.aggBits[a])
+      return __longlong_as_double(s.aggPart[a] == 2 || s.derived[a] ? (long long)(T >> 32)
+                                  : s.aggPart[a] == 1 ? (long long)(T & 0xffffffff) : w0);
     return (double)T;
   }
   if (k == SK_IMIN || k == SK_IMAX) {
-    if (s.nokeys || s.aggBits[a]) {
-      double d;
-      memcpy(&d, &w0, 8);
-      return d;
-    }
-    if (k == SK_IMIN && w0 == 0x7fffffffffffffffll) return bitsToD(0x7ff0000000000000ll);
-    if (k == SK_IMAX && w0 == (long long)0x8000000000000000ull) return bitsToD((long long)0xfff0000000000000ull);
+    if (s.nk == 0 || s.aggBits[a]) return __longlong_as_double(w0);
+    if (k == SK_IMIN && w0 == 0x7fffffffffffffffll) return __longlong_as_double(0x7ff0000000000000ll);
+    if (k == SK_IMAX && w0 == (long long)0x8000000000000000ull) return __longlong_as_double((long long)0xfff0000000000000ull);
     return (double)w0;
   }
-  double d;
-  memcpy(&d, &w0, 8);
-  return d;
+  return __longlong_as_double(w0);
 }
-// colMajor: accs[a * m + j] (compact) else accs[j * na + a] (fetch)
-__global__ void kExactToDouble(const int64_t* exact, int64_t m, DblSpec s, const int16_t* partnerKinds, double* accs,
-                               int colMajor) {
-  for (int64_t j = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; j < m; j += (int64_t)gridDim.x * blockDim.x)
-    for (int a = 0; a < s.na; ++a) {
-      const bool none = s.kind[a] == SK_NONE;
-      const uint8_t sk = none ? (uint8_t)partnerKinds[a] : s.kind[a];
-      accs[colMajor ? a * m + j : j * s.na + a] =
-          slotDouble(s, a, exact[(j * s.na + a) * 2], exact[(j * s.na + a) * 2 + 1], none, sk);
+// Groups p0 .. p0 + n of the result, whose rows are base + list[0 .. n): those within [first, first + limit)
+// to the outputs (all threads of the CTA).
+__device__ __forceinline__ void emitGroups(const ResultSpec& s, const OutSpec& o, int64_t base, const int* list, int n,
+                                           int64_t p0) {
+  const int lo = (int)min((int64_t)n, max((int64_t)0, o.first - p0));
+  const int hi = (int)max((int64_t)lo, min((int64_t)n, o.first + o.limit - p0));
+  const int m = hi - lo;
+  if (m <= 0) return;
+  list += lo;
+  const int64_t at = p0 + lo - o.first;  // output row of the first
+  if (o.keys)
+    for (int t = threadIdx.x; t < m * s.nk; t += blockDim.x) {
+      const int p = o.colRows ? t % m : t / s.nk, k = o.colRows ? t / m : t % s.nk;
+      o.keys[o.colRows ? k * o.colRows + at + p : (at + p) * s.nk + k] = keyOut(s, base + list[p], k);
     }
+  if (o.accs || o.exact)
+    for (int t = threadIdx.x; t < m * s.na; t += blockDim.x) {
+      const int p = o.colRows ? t % m : t / s.na, a = o.colRows ? t / m : t % s.na;
+      long long w0, w1;
+      exactOut(s, base + list[p], a, w0, w1);
+      const int64_t e = (at + p) * s.na + a;
+      if (o.accs) o.accs[o.colRows ? a * o.colRows + at + p : e] = accOut(s, a, w0, w1);
+      if (o.exact) o.exact[2 * e] = w0, o.exact[2 * e + 1] = w1;
+    }
+}
+// Lists the occupied rows of [base, base + rows) in ascending order; returns their number (every thread).
+// rows <= ITERS * blockDim.x, blockDim.x = 32 * WARPS; cnt: [ITERS * WARPS] words of shared memory.
+template <int ITERS, int WARPS>
+__device__ __forceinline__ int listOccupied(const ResultSpec& s, int64_t base, int rows, int* list, int* cnt, int* total) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  unsigned m[ITERS];
+#pragma unroll
+  for (int it = 0; it < ITERS; ++it) {
+    const int r = it * WARPS * 32 + threadIdx.x;
+    m[it] = __ballot_sync(0xffffffffu, r < rows && occupied(s, base + r));
+    if (lane == 0) cnt[it * WARPS + warp] = __popc(m[it]);
+  }
+  __syncthreads();
+  if (warp == 0) {  // exclusive scan of the ITERS * WARPS counts, E of them per lane
+    constexpr int N = ITERS * WARPS, E = (N + 31) / 32;
+    int c[E], sum = 0;
+#pragma unroll
+    for (int e = 0; e < E; ++e) {
+      const int at = lane * E + e;
+      c[e] = at < N ? cnt[at] : 0;
+      sum += c[e];
+    }
+    int incl = sum;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int y = __shfl_up_sync(0xffffffffu, incl, o);
+      if (lane >= o) incl += y;
+    }
+    int run = incl - sum;
+#pragma unroll
+    for (int e = 0; e < E; ++e) {
+      const int at = lane * E + e;
+      if (at < N) cnt[at] = run;
+      run += c[e];
+    }
+    if (lane == 31) *total = incl;
+  }
+  __syncthreads();
+#pragma unroll
+  for (int it = 0; it < ITERS; ++it)
+    if ((m[it] >> lane) & 1u)
+      list[cnt[it * WARPS + warp] + __popc(m[it] & ((1u << lane) - 1u))] = it * WARPS * 32 + threadIdx.x;
+  __syncthreads();
+  return *total;
+}
+__device__ __forceinline__ void writeStatus(const ResultSpec& s, int64_t groups, ws_fetch_status* st) {
+  st->groups = groups;
+  st->overflow = s.mode == 2 && s.err[1] ? 1 : 0;
+  st->error = s.err[0] ? WS_ERR_RANGE : s.err[2] ? WS_ERR_INTERNAL : 0;
+}
+
+// Delivers a result of at most kSmallRows rows.  Nothing but the status is written when the run raised a flag
+// (dense key out of range, staged-copy timeout; hash overflow unless evenOverflowed): the caller reads the
+// status and reruns.
+struct DeliverSpec {
+  ResultSpec r;
+  OutSpec o;
+  ws_fetch_status* st;  // null: not wanted
+  int evenOverflowed;
+};
+__device__ __forceinline__ void deliver(const DeliverSpec& d) {
+  __shared__ int list[kDeliverIters * kDeliverThreads], cnt[kDeliverIters * 32], total;
+  const int g = listOccupied<kDeliverIters, 32>(d.r, 0, (int)d.r.nrows, list, cnt, &total);
+  if (threadIdx.x == 0 && d.st) writeStatus(d.r, g, d.st);
+  if (d.r.err[0] || d.r.err[2] || (d.r.mode == 2 && d.r.err[1] && !d.evenOverflowed)) return;
+  emitGroups(d.r, d.o, 0, list, g, 0);
+}
+__global__ void __launch_bounds__(kDeliverThreads) kDeliver(const __grid_constant__ DeliverSpec d) { deliver(d); }
+__global__ void __launch_bounds__(kDeliverThreads) kDeliverMany(const DeliverSpec* ds) { deliver(ds[blockIdx.x]); }
+
+// Groups of each chunk of kOccChunk result rows; the last CTA turns the counts into offsets (offs[nchunks]:
+// the total) and writes the status (pinned host memory).  *ticket is 0 before and after.
+__global__ void __launch_bounds__(kOccThreads) kOccCount(const __grid_constant__ ResultSpec s, int64_t* offs,
+                                                         int64_t nchunks, unsigned* ticket, ws_fetch_status* st) {
+  __shared__ int64_t wsum[kOccThreads / 32];
+  __shared__ bool amLast;
+  const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
+  const int64_t c0 = (int64_t)blockIdx.x * kOccChunk;
+  int c = 0;
+#pragma unroll
+  for (int it = 0; it < kOccChunk / kOccThreads; ++it) {
+    const int64_t i = c0 + it * kOccThreads + t;
+    c += i < s.nrows && occupied(s, i);
+  }
+  c = __reduce_add_sync(0xffffffffu, c);
+  if (lane == 0) wsum[warp] = c;
+  __syncthreads();
+  if (t == 0) {
+    int64_t sum = 0;
+    for (int w = 0; w < kOccThreads / 32; ++w) sum += wsum[w];
+    offs[blockIdx.x] = sum;
+    __threadfence();
+    amLast = atomicAdd(ticket, 1u) == gridDim.x - 1;
+  }
+  __syncthreads();
+  if (!amLast) return;
+  __threadfence();
+  constexpr int E = 8;  // counts per thread and step
+  int64_t run = 0;
+  for (int64_t b = 0; b < nchunks; b += kOccThreads * E) {
+    int64_t v[E], sum = 0;
+#pragma unroll
+    for (int e = 0; e < E; ++e) {
+      const int64_t i = b + t * E + e;
+      v[e] = i < nchunks ? __ldcg((const long long*)offs + i) : 0;
+      sum += v[e];
+    }
+    int64_t incl = sum;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int64_t y = __shfl_up_sync(0xffffffffu, incl, o);
+      if (lane >= o) incl += y;
+    }
+    __syncthreads();
+    if (lane == 31) wsum[warp] = incl;
+    __syncthreads();
+    int64_t before = 0, all = 0;
+    for (int w = 0; w < kOccThreads / 32; ++w) {
+      if (w < warp) before += wsum[w];
+      all += wsum[w];
+    }
+    int64_t at = run + before + incl - sum;
+#pragma unroll
+    for (int e = 0; e < E; ++e) {
+      const int64_t i = b + t * E + e;
+      if (i < nchunks) offs[i] = at;
+      at += v[e];
+    }
+    run += all;
+  }
+  if (t == 0) {
+    offs[nchunks] = run;
+    *ticket = 0;
+    writeStatus(s, run, st);
+  }
+}
+// Groups of chunk blockIdx.x (the groups from offs[chunk] on) to the outputs; nothing when the run raised a
+// flag (as kDeliver).
+__global__ void __launch_bounds__(kOccThreads) kEmitChunks(const __grid_constant__ ResultSpec s,
+                                                           const __grid_constant__ OutSpec o, const int64_t* offs,
+                                                           int evenOverflowed) {
+  constexpr int kIters = kOccChunk / kOccThreads, kWarps = kOccThreads / 32;
+  __shared__ int list[kOccChunk], cnt[kIters * kWarps], total;
+  if (s.err[0] || s.err[2] || (s.mode == 2 && s.err[1] && !evenOverflowed)) return;
+  const int64_t p0 = offs[blockIdx.x], p1 = offs[blockIdx.x + 1];
+  if (p0 == p1 || p1 <= o.first || p0 >= o.first + o.limit) return;  // none of this chunk's groups
+  const int64_t base = (int64_t)blockIdx.x * kOccChunk;
+  const int n = listOccupied<kIters, kWarps>(s, base, (int)min((int64_t)kOccChunk, s.nrows - base), list, cnt, &total);
+  emitGroups(s, o, base, list, n, p0);
+}
+// The status alone (offsets known from an earlier range of the same run).
+__global__ void kFetchStatus(const __grid_constant__ ResultSpec s, const int64_t* total, ws_fetch_status* st) {
+  writeStatus(s, *total, st);
 }
 
 }  // namespace
@@ -439,23 +486,23 @@ struct ws_aggregator {
   int batchesDone = 0, windows = 0;
   DBuf<u64> rows;
   DBuf<double> tkeys;
-  DBuf<uint8_t> ctl;  // [count u64][err int x3][pad][ticket u32]
-  bool fetched = false;
+  // control words (kCtlWords u64 after the rows): [count u64][err int x3][occTicket u32][ticket u32][pad]
+  uint8_t* ctl() { return (uint8_t*)(rows.p + nrows() * lay.rw); }
   std::vector<int64_t> hi;
-  int64_t lastGroups = -1;
-  // groups compacted on the device by the last fetch (reused by the copy after a size query, until
-  // the next run): keys and engine-format doubles row-major, exact words [g][na][2]
-  int64_t cachedGroups = -1;
-  DBuf<double> cachedKeys, cachedAccs;
-  DBuf<int64_t> cachedExact;
-  std::vector<int64_t> cachedHi;
-  // groups before each chunk of kOccChunk result rows (ws_agg_fetch_async), until the next run
-  DBuf<int64_t> fetchOffs;
-  bool fetchOffsValid = false;
+  // What the last fetch learned of the run's result, until the next run: the status (flags, groups), of a small
+  // result also its groups in host memory (keys and engine-format doubles row-major, exact words [g][na][2]),
+  // of a larger one the groups before each chunk of kOccChunk result rows.
+  bool statusKnown = false, groupsOnHost = false, offsKnown = false;
+  ws_fetch_status status{};
+  std::vector<double> hostKeys, hostAccs;
+  std::vector<int64_t> hostExact;
+  DBuf<int64_t> offs;
+  void newRun() { statusKnown = groupsOnHost = offsKnown = false; }
 
-  u64* count() { return (u64*)ctl.p; }
-  int* err() { return (int*)(ctl.p + 8); }
-  unsigned* ticket() { return (unsigned*)(ctl.p + 24); }
+  u64* count() { return (u64*)ctl(); }
+  int* err() { return (int*)(ctl() + 8); }
+  unsigned* occTicket() { return (unsigned*)(ctl() + 20); }
+  unsigned* ticket() { return (unsigned*)(ctl() + 24); }
   int64_t nrows() const { return isDense ? dense.G : plan.nkeys ? cap + 1 : 1; }
 };
 
@@ -488,21 +535,23 @@ static RowTemplate rowTemplate(const SlotLayout& lay) {
   return t;
 }
 
-// Result rows to their identities (hash rows empty) and the control words (count, flags, ticket) to 0.
-static void aggResetRows(ws_aggregator& A) {
-  const int64_t nr = A.nrows();
+static FillSpec fillSpec(ws_aggregator& A) {
   const int64_t emptyRows = A.plan.nkeys && !A.isDense ? A.cap : 0;
-  WS_LAUNCH(kFillRows, gridFor(nr), 256, 0, A.rows.p, nr, A.lay.rw, rowTemplate(A.lay), emptyRows);
-  WS_CK(cudaMemsetAsync(A.ctl.p, 0, 32, stream()));
+  return FillSpec{A.rows.p, A.nrows() * A.lay.rw, emptyRows * A.lay.rw, A.lay.rw, (u64*)A.ctl(), rowTemplate(A.lay)};
+}
+
+// Result rows to their identities (hash rows empty) and the control words (count, flags, tickets) to 0.
+static void aggResetRows(ws_aggregator& A) {
+  const FillSpec f = fillSpec(A);
+  WS_LAUNCH(kFillRows, gridFor(f.words, 256, 16), 256, 0, f);
 }
 
 static void aggInitRows(ws_aggregator& A) {
   const int64_t nr = A.nrows();
-  A.rows = DBuf<u64>(nr * A.lay.rw);
+  A.rows = DBuf<u64>(nr * A.lay.rw + kCtlWords);
   if (A.plan.nkeys && !A.isDense) {
     A.tkeys = DBuf<double>((A.cap + 1) * std::max(A.plan.nkeys, 1));
   }
-  A.ctl = DBuf<uint8_t>(32);
   aggResetRows(A);
 }
 
@@ -549,10 +598,7 @@ struct PreparedScan {
 static void aggRun(ws_aggregator& A, const ws_expr_env& env, const ws_jit_program* jit, PreparedScan* prep = nullptr) {
   const int nb = (int)A.bn.size();
   if (nb == 0) return;
-  A.fetched = false;
-  A.lastGroups = -1;
-  A.cachedGroups = -1;
-  A.fetchOffsValid = false;
+  A.newRun();
   const bool useJit = jit && jit->state.load() == 1 && planCovers(env, nb, A.ncols, A.bcols.data());
   if (!useJit && (A.plan.naggs > WS_INTERP_AGGS || A.plan.nkeys > WS_INTERP_KEYS))
     throw Error("this aggregation needs a compiled plan (more than 16 aggregates or 4 GROUP BY keys); codegen failed or is off", WS_ERR_PLAN);
@@ -786,31 +832,25 @@ static TuneChoice tuneScan(ws_aggregator& A, const std::string& key, const std::
   return best;
 }
 
-// Occupied row indices of the result rows (ascending), on the device; returns the count.
-static int64_t aggCompactIdx(ws_aggregator& A, DBuf<int64_t>& idx) {
-  const int64_t nr = A.nrows();
-  OccSpec s{A.lay.rw, A.isDense ? 1 : 2, A.lay.woff[0], A.cap};
-  const int64_t nchunks = (nr + kOccChunk - 1) / kOccChunk;
-  DBuf<int64_t> counts(nchunks + 1);
-  WS_LAUNCH(kOccCount, (unsigned)nchunks, 256, 0, A.rows.p, nr, s, counts.p);
-  WS_LAUNCH(kScanExclusive, 1, 1024, 0, counts.p, nchunks);
-  int64_t g = 0;
-  d2hSync(&g, counts.p + nchunks, 8);
-  idx = DBuf<int64_t>(std::max<int64_t>(g, 1));
-  if (g) WS_LAUNCH(kOccWrite, (unsigned)nchunks, 256, 0, A.rows.p, nr, s, counts.p, idx.p);
-  return g;
-}
-
-static EmitSpec emitSpec(const ws_aggregator& A) {
-  EmitSpec s{};
-  s.nk = A.plan.nkeys;
-  s.na = A.plan.naggs;
+static ResultSpec resultSpec(ws_aggregator& A) {
+  ResultSpec s{};
+  s.rows = A.rows.p;
+  s.nrows = A.nrows();
+  s.cap = A.cap;
+  s.err = A.err();
+  s.tkeys = A.tkeys.p;
   s.rw = A.lay.rw;
   s.mode = A.plan.nkeys == 0 ? 0 : A.isDense ? 1 : 2;
+  s.cnt0 = A.lay.woff[0];
+  s.nk = A.plan.nkeys;
+  s.na = A.plan.naggs;
   for (int a = 0; a < s.na; ++a) {
-    s.kind[a] = A.lay.kind[a];
-    s.woff[a] = (int16_t)A.lay.woff[a];
-    s.partner[a] = (int16_t)A.lay.partner[a];
+    s.derived[a] = A.lay.kind[a] == SK_NONE;
+    const int src = s.derived[a] ? A.lay.partner[a] : a;
+    s.kind[a] = A.lay.kind[src];
+    s.woff[a] = (int16_t)A.lay.woff[src];
+    s.aggBits[a] = A.plan.aggBits[a];
+    s.aggPart[a] = A.plan.aggPart[a];
   }
   for (int k = 0; k < s.nk; ++k) {
     s.keyInt[k] = A.plan.keyInt[k];
@@ -818,29 +858,80 @@ static EmitSpec emitSpec(const ws_aggregator& A) {
     s.range[k] = A.isDense ? A.dense.range[k] : 1;
     s.stride[k] = A.isDense ? A.dense.stride[k] : 1;
   }
-  s.tkeys = A.tkeys.p;
-  s.cap = A.cap;
   return s;
 }
 
-static DblSpec dblSpec(const ws_aggregator& A) {
-  DblSpec s{};
-  s.na = A.plan.naggs;
-  s.nokeys = A.plan.nkeys == 0;
-  for (int a = 0; a < s.na; ++a) {
-    s.kind[a] = A.lay.kind[a];
-    s.aggBits[a] = A.plan.aggBits[a];
-    s.aggPart[a] = A.plan.aggPart[a];
+// Pinned and mapped memory that small results are delivered into, one block per thread (its size is bounded
+// by kHostResultBytes; freed when the thread ends).  Its contents are copied out before the call returns.
+constexpr size_t kHostResultBytes = 1u << 20;
+static uint8_t* hostResult() {
+  struct Block {
+    uint8_t* p = nullptr;
+    ~Block() {
+      if (p) cudaFreeHost(p);
+    }
+  };
+  static thread_local Block b;
+  if (!b.p) WS_CK(cudaHostAlloc((void**)&b.p, kHostResultBytes, cudaHostAllocMapped));
+  return b.p;
+}
+template <class T>
+static T* mappedPtr(T* host) {
+  void* d = nullptr;
+  WS_CK(cudaHostGetDevicePointer(&d, (void*)host, 0));
+  return (T*)d;
+}
+
+constexpr size_t kStatusBytes = 64;  // the status at the start of a host result block
+// A result delivered whole into the thread's host block: few rows, all of whose groups fit it.
+static bool smallResult(const ws_aggregator& A) {
+  return A.nrows() <= kSmallRows &&
+         kStatusBytes + (size_t)A.nrows() * 8 * (size_t)(A.plan.nkeys + 3 * A.plan.naggs) <= kHostResultBytes;
+}
+
+// The run's status (flags and number of groups) on the host: a small result is delivered whole, a larger
+// one's chunks are counted.  One wait.
+static const ws_fetch_status& learnStatus(ws_aggregator& A) {
+  if (A.statusKnown) return A.status;
+  uint8_t* h = hostResult();
+  uint8_t* d = mappedPtr(h);
+  const size_t nk = (size_t)A.plan.nkeys, na = (size_t)A.plan.naggs, nr = (size_t)A.nrows();
+  const size_t oKeys = kStatusBytes, oAccs = oKeys + 8 * nk * nr, oExact = oAccs + 8 * na * nr;
+  const bool small = smallResult(A);
+  if (small) {
+    DeliverSpec ds{resultSpec(A),
+                   {nk ? (double*)(d + oKeys) : nullptr, (double*)(d + oAccs), (long long*)(d + oExact), 0, (int64_t)nr, 0},
+                   (ws_fetch_status*)d, 1};
+    WS_LAUNCH(kDeliver, 1, kDeliverThreads, 0, ds);
+  } else {
+    const int64_t nchunks = ((int64_t)nr + kOccChunk - 1) / kOccChunk;
+    A.offs = DBuf<int64_t>(nchunks + 1);
+    WS_LAUNCH(kOccCount, (unsigned)nchunks, kOccThreads, 0, resultSpec(A), A.offs.p, nchunks, A.occTicket(),
+              (ws_fetch_status*)d);
+    A.offsKnown = true;
   }
-  return s;
+  sync();
+  memcpy(&A.status, h, sizeof A.status);
+  if (small && !A.status.error) {
+    const size_t g = (size_t)A.status.groups;
+    A.hostKeys.assign((const double*)(h + oKeys), (const double*)(h + oKeys) + g * nk);
+    A.hostAccs.assign((const double*)(h + oAccs), (const double*)(h + oAccs) + g * na);
+    A.hostExact.assign((const int64_t*)(h + oExact), (const int64_t*)(h + oExact) + g * na * 2);
+    A.groupsOnHost = true;
+  }
+  A.statusKnown = true;
+  return A.status;
 }
 
-static void checkFlags(ws_aggregator& A, bool* overflow) {
-  int e[3] = {0, 0, 0};
-  d2hSync(e, A.err(), 12);
-  if (e[0]) throw Error("dense GROUP BY key outside its declared range", WS_ERR_RANGE);
-  if (e[2]) throw Error("a staged tile copy did not complete in time", WS_ERR_INTERNAL);
-  if (overflow) *overflow = e[1] != 0;
+static void throwFlags(const ws_fetch_status& st) {
+  if (st.error == WS_ERR_RANGE) throw Error("dense GROUP BY key outside its declared range", WS_ERR_RANGE);
+  if (st.error) throw Error("a staged tile copy did not complete in time", WS_ERR_INTERNAL);
+}
+
+// Queues the groups of a counted result (offs known) to device or mapped memory.
+static void emitChunks(ws_aggregator& A, const int64_t* offs, const OutSpec& o, bool evenOverflowed) {
+  WS_LAUNCH(kEmitChunks, (unsigned)((A.nrows() + kOccChunk - 1) / kOccChunk), kOccThreads, 0, resultSpec(A), o, offs,
+            evenOverflowed ? 1 : 0);
 }
 
 // One multi-query scan over prepared queries (ws_agg_run_many, ws_exec_group_*): the kernel of the
@@ -1013,9 +1104,16 @@ int64_t ws_agg_capacity(const ws_aggregator* A) { return A->cap; }
 
 int ws_agg_overflowed(ws_aggregator* A, int* out) {
   return guardedCall([&] {
-    bool o = false;
-    checkFlags(*A, &o);
-    *out = A->plan.nkeys && !A->isDense && o ? 1 : 0;
+    if (smallResult(*A) || A->statusKnown) {  // the groups come along: a fetch usually follows
+      const ws_fetch_status& st = learnStatus(*A);
+      throwFlags(st);
+      *out = st.overflow;
+      return;
+    }
+    int e[3] = {0, 0, 0};
+    d2hSync(e, A->err(), 12);
+    throwFlags(ws_fetch_status{0, 0, e[0] ? WS_ERR_RANGE : e[2] ? WS_ERR_INTERNAL : 0});
+    *out = A->plan.nkeys && !A->isDense && e[1] ? 1 : 0;
   });
 }
 
@@ -1026,8 +1124,7 @@ int ws_agg_group_count(ws_aggregator* A, int64_t* out) {
       return;
     }
     if (A->isDense) {
-      DBuf<int64_t> idx;
-      *out = aggCompactIdx(*A, idx);
+      *out = learnStatus(*A).groups;
       return;
     }
     u64 c = 0;
@@ -1039,53 +1136,37 @@ int ws_agg_group_count(ws_aggregator* A, int64_t* out) {
 int ws_agg_fetch(ws_aggregator* A, int64_t max_groups, double* keys, double* accs, int64_t* exact, int64_t* ngroups) {
   return guardedCall([&] {
     const int nk = A->plan.nkeys, na = A->plan.naggs;
-    if (A->cachedGroups < 0) {  // compact and convert on the device once; the copy after a size query reuses it
-      checkFlags(*A, nullptr);
-      DBuf<int64_t> idx;
-      const int64_t g = nk ? aggCompactIdx(*A, idx) : 1;
-      A->cachedKeys = DBuf<double>(std::max<int64_t>(g * nk, 1));
-      A->cachedExact = DBuf<int64_t>(std::max<int64_t>(g * na * 2, 1));
-      A->cachedAccs = DBuf<double>(std::max<int64_t>(g * na, 1));
-      if (g) {
-        WS_LAUNCH(kEmit, gridFor(g), 256, 0, A->rows.p, nk ? idx.p : nullptr, g, emitSpec(*A), A->cachedKeys.p,
-                  A->cachedExact.p, 0);
-        DBuf<int16_t> pk(WS_MAX_AGGS);
-        int16_t* st = (int16_t*)pinnedStage(2 * WS_MAX_AGGS);
-        for (int a = 0; a < WS_MAX_AGGS; ++a) st[a] = a < na ? A->lay.kind[A->lay.partner[a]] : 0;
-        h2dAsync(pk.p, st, 2 * WS_MAX_AGGS);
-        stageCopied();
-        WS_LAUNCH(kExactToDouble, gridFor(g), 256, 0, A->cachedExact.p, g, dblSpec(*A), pk.p, A->cachedAccs.p, 0);
-      }
-      A->cachedHi.assign(na, 0);
-      if (!nk) {  // high words of exact no-key integer sums (sumHigh)
-        std::vector<int64_t> ex(2 * na);
-        d2hSync(ex.data(), A->cachedExact.p, 16 * na);
-        for (int a = 0; a < na; ++a) {
-          const uint8_t k = A->lay.kind[a] == SK_NONE ? A->lay.kind[A->lay.partner[a]] : A->lay.kind[a];
-          A->cachedHi[a] = k == SK_ISUM ? ex[2 * a + 1] : 0;
-        }
-      } else {
-        sync();
-      }
-      A->cachedGroups = g;
-    }
-    const int64_t g = A->cachedGroups;
+    const ws_fetch_status& st = learnStatus(*A);
+    throwFlags(st);
+    const int64_t g = st.groups;
     *ngroups = g;
     if (g > max_groups) throw Error("output buffer too small for " + std::to_string(g) + " groups", WS_ERR_SIZE);
-    if (g) {
-      if (nk && keys) d2hLarge(keys, A->cachedKeys.p, sizeof(double) * g * nk);
-      if (accs) d2hLarge(accs, A->cachedAccs.p, sizeof(double) * g * na);
-      if (exact) d2hLarge(exact, A->cachedExact.p, sizeof(int64_t) * g * na * 2);
+    if (!nk) keys = nullptr;
+    if (A->groupsOnHost) {
+      if (keys) memcpy(keys, A->hostKeys.data(), sizeof(double) * g * nk);
+      if (accs) memcpy(accs, A->hostAccs.data(), sizeof(double) * g * na);
+      if (exact) memcpy(exact, A->hostExact.data(), sizeof(int64_t) * g * na * 2);
+    } else if (g && (keys || accs || exact)) {
+      DBuf<double> dk(keys ? g * nk : 0), da(accs ? g * na : 0);
+      DBuf<int64_t> dx(exact ? g * na * 2 : 0);
+      emitChunks(*A, A->offs.p, OutSpec{dk.p, da.p, (long long*)dx.p, 0, g, 0}, true);
+      if (keys) d2hLarge(keys, dk.p, sizeof(double) * g * nk);
+      if (accs) d2hLarge(accs, da.p, sizeof(double) * g * na);
+      if (exact) d2hLarge(exact, dx.p, sizeof(int64_t) * g * na * 2);
     }
-    A->hi = A->cachedHi;
-    A->fetched = true;
+    A->hi.assign(na, 0);
+    if (!nk && A->groupsOnHost)  // high words of exact no-key integer sums (sumHigh)
+      for (int a = 0; a < na; ++a) {
+        const uint8_t k = A->lay.kind[a] == SK_NONE ? A->lay.kind[A->lay.partner[a]] : A->lay.kind[a];
+        A->hi[a] = k == SK_ISUM ? A->hostExact[2 * a + 1] : 0;
+      }
   });
 }
 
 int ws_agg_fetch_async(ws_aggregator* A, int64_t first_group, int64_t max_groups, double* keys, int64_t* exact,
                        ws_fetch_status* status) {
   return guardedCall([&] {
-    const int nk = A->plan.nkeys, na = A->plan.naggs;
+    const int nk = A->plan.nkeys;
     auto mapped = [](void* h, const char* what) -> void* {
       if (!h) throw Error(std::string("fetch_async: ") + what + " is null", WS_ERR_ARG);
       cudaPointerAttributes at{};
@@ -1099,25 +1180,20 @@ int ws_agg_fetch_async(ws_aggregator* A, int64_t first_group, int64_t max_groups
     double* dk = nk ? (double*)mapped(keys, "keys") : nullptr;
     auto* dx = (long long*)mapped(exact, "exact");
     if (first_group < 0 || max_groups < 0) throw Error("fetch_async: negative group range", WS_ERR_ARG);
-    const int64_t nr = A->nrows();
-    OccSpec o{A->lay.rw, nk == 0 ? 0 : A->isDense ? 1 : 2, A->lay.woff[0], A->cap};
-    const int64_t nchunks = (nr + kOccChunk - 1) / kOccChunk;
-    if (!A->fetchOffsValid) {  // group offsets per chunk, kept for the later ranges of the same run
-      A->fetchOffs = DBuf<int64_t>(nchunks + 1);
-      WS_LAUNCH(kOccCount, (unsigned)nchunks, 256, 0, A->rows.p, nr, o, A->fetchOffs.p);
-      WS_LAUNCH(kScanExclusive, 1, 1024, 0, A->fetchOffs.p, nchunks);
-      A->fetchOffsValid = true;
+    const OutSpec o{dk, nullptr, dx, first_group, max_groups, 0};
+    if (A->nrows() <= kSmallRows) {
+      WS_LAUNCH(kDeliver, 1, kDeliverThreads, 0, DeliverSpec{resultSpec(*A), o, st, 0});
+      return;
     }
-    const int64_t* counts = A->fetchOffs.p;
-    WS_LAUNCH(kFetchStatus, 1, 1, 0, counts + nchunks, A->err(), o.mode == 2 ? 1 : 0, st);
-    if (max_groups == 0) return;
-    // sub-tile rows: staging of at most 32 KB, a multiple of 32 rows
-    const int rowBytes = 8 * (nk + 2 * na);
-    const int threads = std::max(32, std::min(256, (32768 / rowBytes) & ~31));
-    WS_LAUNCH(kOccEmitHost, (unsigned)nchunks, threads, (size_t)threads * rowBytes, A->rows.p, nr, o, emitSpec(*A),
-              counts, nchunks, A->err(), first_group, max_groups, dk, dx);
-    A->cachedGroups = -1;
-    A->fetched = true;
+    const int64_t nchunks = (A->nrows() + kOccChunk - 1) / kOccChunk;
+    if (!A->offsKnown) {  // group offsets per chunk, kept for the later ranges of the same run
+      A->offs = DBuf<int64_t>(nchunks + 1);
+      WS_LAUNCH(kOccCount, (unsigned)nchunks, kOccThreads, 0, resultSpec(*A), A->offs.p, nchunks, A->occTicket(), st);
+      A->offsKnown = true;
+    } else {
+      WS_LAUNCH(kFetchStatus, 1, 1, 0, resultSpec(*A), A->offs.p + nchunks, st);
+    }
+    if (max_groups) emitChunks(*A, A->offs.p, o, false);
   });
 }
 
@@ -1152,27 +1228,23 @@ struct ws_executor {
 };
 
 namespace {
+OutSpec execOut(ws_executor& X) {
+  return OutSpec{X.A->plan.nkeys ? mappedPtr(X.keys) : nullptr, nullptr, (long long*)mappedPtr(X.exact), 0, X.maxGroups, 0};
+}
 // Queues on this thread's stream the part of a prepared query after its scan: compaction of the
-// result rows, the status word and the groups written into the executor's pinned memory.
-void queueExecTail(ws_executor& X) {
+// result rows, the status word and the groups written into the executor's pinned memory.  Returns the
+// kernels queued.
+int queueExecTail(ws_executor& X) {
   ws_aggregator& A = *X.A;
-  const int nk = A.plan.nkeys, na = A.plan.naggs;
-  double* dk = nullptr;
-  long long* dx = nullptr;
-  ws_fetch_status* dst = nullptr;
-  WS_CK(cudaHostGetDevicePointer((void**)&dk, X.keys, 0));
-  WS_CK(cudaHostGetDevicePointer((void**)&dx, X.exact, 0));
-  WS_CK(cudaHostGetDevicePointer((void**)&dst, X.st, 0));
-  const int64_t nr = A.nrows();
-  const OccSpec o{A.lay.rw, nk == 0 ? 0 : A.isDense ? 1 : 2, A.lay.woff[0], A.cap};
-  const int64_t nchunks = (nr + kOccChunk - 1) / kOccChunk;
-  const int rowBytes = 8 * (nk + 2 * na);
-  const int threads = std::max(32, std::min(256, (32768 / rowBytes) & ~31));
-  WS_LAUNCH(kOccCount, (unsigned)nchunks, 256, 0, A.rows.p, nr, o, X.offs.p);
-  WS_LAUNCH(kScanExclusive, 1, 1024, 0, X.offs.p, nchunks);
-  WS_LAUNCH(kFetchStatus, 1, 1, 0, X.offs.p + nchunks, A.err(), o.mode == 2 ? 1 : 0, dst);
-  WS_LAUNCH(kOccEmitHost, (unsigned)nchunks, threads, (size_t)threads * rowBytes, A.rows.p, nr, o, emitSpec(A), X.offs.p,
-            nchunks, A.err(), (int64_t)0, X.maxGroups, dk, dx);
+  ws_fetch_status* st = mappedPtr(X.st);
+  if (A.nrows() <= kSmallRows) {
+    WS_LAUNCH(kDeliver, 1, kDeliverThreads, 0, DeliverSpec{resultSpec(A), execOut(X), st, 0});
+    return 1;
+  }
+  const int64_t nchunks = (A.nrows() + kOccChunk - 1) / kOccChunk;
+  WS_LAUNCH(kOccCount, (unsigned)nchunks, kOccThreads, 0, resultSpec(A), X.offs.p, nchunks, A.occTicket(), st);
+  emitChunks(A, X.offs.p, execOut(X), false);
+  return 2;
 }
 
 uint64_t codeDigest(const ws_expr_env& env) {
@@ -1241,8 +1313,7 @@ int ws_exec_create(const ws_agg_plan* plan, int64_t capacity, const ws_dense_spe
         X->scanNode = deps[0];
         ++X->kernels;
       }
-      queueExecTail(*X);
-      X->kernels += 4;
+      X->kernels += queueExecTail(*X);
       capturing = false;
       WS_CK(cudaStreamEndCapture(cs, &X->graph));
       WS_CK(cudaGraphInstantiate(&X->exec, X->graph, 0));
@@ -1306,6 +1377,7 @@ struct ws_exec_group {
   uint8_t* stage = nullptr;  // pinned: [Launch per live query][CTA starts]
   size_t stageBytes = 0;
   ws::DBuf<uint8_t> dl;      // the device copy the scan reads
+  ws::DBuf<uint8_t> specs;   // the queries' reset specs, then the delivery specs of those with small results
   cudaGraph_t graph = nullptr;
   cudaGraphExec_t exec = nullptr;
   cudaEvent_t done = nullptr;  // the last run's end: its copy of `stage` has been made
@@ -1351,6 +1423,19 @@ int ws_exec_group_create(ws_executor* const* xs, int n, const ws_jit_program* ji
       G->dl = DBuf<uint8_t>((int64_t)G->stageBytes);
     }
     WS_CK(cudaEventCreateWithFlags(&G->done, cudaEventDisableTiming));
+    // every query's rows are reset by one launch, and the small results delivered by one (a CTA each)
+    std::vector<FillSpec> fills;
+    std::vector<DeliverSpec> small;
+    int64_t fillWords = 1;
+    for (ws_executor* X : G->xs) {
+      fills.push_back(fillSpec(*X->A));
+      fillWords = std::max(fillWords, fills.back().words);
+      if (X->A->nrows() <= kSmallRows) small.push_back(DeliverSpec{resultSpec(*X->A), execOut(*X), mappedPtr(X->st), 0});
+    }
+    const size_t fillBytes = fills.size() * sizeof(FillSpec), smallBytes = small.size() * sizeof(DeliverSpec);
+    G->specs = DBuf<uint8_t>((int64_t)(fillBytes + smallBytes));
+    WS_CK(cudaMemcpyAsync(G->specs.p, fills.data(), fillBytes, cudaMemcpyHostToDevice, stream()));
+    WS_CK(cudaMemcpyAsync(G->specs.p + fillBytes, small.data(), smallBytes, cudaMemcpyHostToDevice, stream()));
     sync();  // allocations done before the capture starts
     cudaStream_t cs = nullptr;
     WS_CK(cudaStreamCreateWithFlags(&cs, cudaStreamNonBlocking));
@@ -1362,11 +1447,9 @@ int ws_exec_group_create(ws_executor* const* xs, int n, const ws_jit_program* ji
     try {
       WS_CK(cudaStreamBeginCapture(cs, cudaStreamCaptureModeThreadLocal));
       capturing = true;
-      for (ws_executor* X : G->xs) aggResetRows(*X->A);
+      WS_LAUNCH(kFillRowsMany, dim3(gridFor(fillWords), (unsigned)fills.size()), 256, 0, (const FillSpec*)G->specs.p);
       if (nl) {
         WS_CK(cudaMemcpyAsync(G->dl.p, G->stage, G->stageBytes, cudaMemcpyHostToDevice, cs));
-        for (const Launch& L : mp.L)
-          if (L.ticket) WS_CK(cudaMemsetAsync(L.ticket, 0, 4, cs));
         MultiLaunch M{(const Launch*)G->dl.p, (const int*)(G->dl.p + launchBytes), (int)nl};
         allowDynamicSmem(mp.f, mp.smem);
         void* args[] = {(void*)&M};
@@ -1374,7 +1457,11 @@ int ws_exec_group_create(ws_executor* const* xs, int n, const ws_jit_program* ji
                                   (CUstream)cs, args, nullptr));
         countLaunch();
       }
-      for (ws_executor* X : G->xs) queueExecTail(*X);
+      if (!small.empty())
+        WS_LAUNCH(kDeliverMany, (unsigned)small.size(), kDeliverThreads, 0,
+                  (const DeliverSpec*)(G->specs.p + fillBytes));
+      for (ws_executor* X : G->xs)
+        if (X->A->nrows() > kSmallRows) queueExecTail(*X);
       capturing = false;
       WS_CK(cudaStreamEndCapture(cs, &G->graph));
       WS_CK(cudaGraphInstantiate(&G->exec, G->graph, 0));
@@ -1453,20 +1540,17 @@ int ws_agg_sum_high(const ws_aggregator* A, int64_t* out) {
 
 int ws_agg_compact(ws_aggregator* A, double** keys, double** accs, int64_t* ngroups) {
   return guardedCall([&] {
-    checkFlags(*A, nullptr);
     const int nk = A->plan.nkeys, na = A->plan.naggs;
-    DBuf<int64_t> idx;
-    const int64_t g = nk ? aggCompactIdx(*A, idx) : 1;
+    const ws_fetch_status& st = learnStatus(*A);
+    throwFlags(st);
+    const int64_t g = st.groups;
     DBuf<double> dk(std::max<int64_t>(g * nk, 1)), da(std::max<int64_t>(g * na, 1));
-    DBuf<int64_t> dx(std::max<int64_t>(g * na * 2, 1));
-    DBuf<int16_t> pk(WS_MAX_AGGS);
-    if (g) {
-      WS_LAUNCH(kEmit, gridFor(g), 256, 0, A->rows.p, nk ? idx.p : nullptr, g, emitSpec(*A), dk.p, dx.p, 1);
-      int16_t* st = (int16_t*)pinnedStage(2 * WS_MAX_AGGS);
-      for (int a = 0; a < WS_MAX_AGGS; ++a) st[a] = a < na ? A->lay.kind[A->lay.partner[a]] : 0;
-      h2dAsync(pk.p, st, 2 * WS_MAX_AGGS);
-      stageCopied();
-      WS_LAUNCH(kExactToDouble, gridFor(g), 256, 0, dx.p, g, dblSpec(*A), pk.p, da.p, 1);
+    if (g && A->groupsOnHost) {
+      // a small result again, now into device memory
+      WS_LAUNCH(kDeliver, 1, kDeliverThreads, 0,
+                DeliverSpec{resultSpec(*A), {nk ? dk.p : nullptr, da.p, nullptr, 0, g, g}, nullptr, 1});
+    } else if (g) {
+      emitChunks(*A, A->offs.p, OutSpec{nk ? dk.p : nullptr, da.p, nullptr, 0, g, g}, true);
     }
     *keys = dk.release();
     *accs = da.release();
