@@ -92,6 +92,13 @@ WS_DI i64 imul32w(i64 a, i64 b, unsigned& wide) {
   wide |= ((unsigned)((u64)a >> 32) ^ (unsigned)((int)a >> 31)) | ((unsigned)((u64)b >> 32) ^ (unsigned)((int)b >> 31));
   return (i64)(int)a * (i64)(int)b;
 }
+// Non-zero when v does not fit in int32.
+WS_DI unsigned wide32(i64 v) { return (unsigned)((u64)v >> 32) ^ (unsigned)((int)v >> 31); }
+// High word of the magnitude of an integer SUM argument (see sumMagnitude in ws_kern.cuh).
+WS_DI unsigned magHigh(i64 v) {
+  const unsigned hi = (unsigned)((u64)v >> 32);
+  return hi ^ (unsigned)((int)hi >> 31);
+}
 WS_DI i64 imulf(i64 a, i64 b, unsigned& of) {
   if (a == (i64)(int)a && b == (i64)(int)b) return (i64)(int)a * (i64)(int)b;  // 32 x 32 bits: exact
   const i64 r = (i64)((u64)a * (u64)b);
@@ -306,6 +313,75 @@ WS_DI unsigned ldg1(const void* p) {
   unsigned v;
   asm volatile("ld.global.nc.L1::no_allocate.u32 %0, [%1];" : "=r"(v) : "l"(p));
   return v;
+}
+
+// Four consecutive rows of a column as stored (1, 2, 4 or 8 bytes per row), packed in 32-bit words.  The
+// evaluators of raw and hinted columns fetch every column this way before any value is decoded, so that a
+// thread's loads are all in flight together.  `fast`, nv: as below.
+WS_DI void fetch4(int (&r)[8], const unsigned char* p, bool fast, int nv) {
+  if (fast) {
+    const int4 a = ldg4(p), b = ldg4(p + 16);
+    r[0] = a.x, r[1] = a.y, r[2] = a.z, r[3] = a.w, r[4] = b.x, r[5] = b.y, r[6] = b.z, r[7] = b.w;
+  } else {
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const u64 v = i < nv ? __ldg((const u64*)p + i) : 0ull;
+      r[2 * i] = (int)v, r[2 * i + 1] = (int)(v >> 32);
+    }
+  }
+}
+WS_DI void fetch4(int (&r)[4], const unsigned char* p, bool fast, int nv) {
+  if (fast) {
+    const int4 a = ldg4(p);
+    r[0] = a.x, r[1] = a.y, r[2] = a.z, r[3] = a.w;
+  } else {
+#pragma unroll
+    for (int i = 0; i < 4; ++i) r[i] = i < nv ? __ldg((const int*)p + i) : 0;
+  }
+}
+WS_DI void fetch4(int (&r)[2], const unsigned char* p, bool fast, int nv) {
+  if (fast) {
+    const int2 a = ldg2(p);
+    r[0] = a.x, r[1] = a.y;
+  } else {
+    unsigned c[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) c[i] = i < nv ? (unsigned)__ldg((const unsigned short*)p + i) : 0u;
+    r[0] = (int)(c[0] | c[1] << 16), r[1] = (int)(c[2] | c[3] << 16);
+  }
+}
+WS_DI void fetch4(int (&r)[1], const unsigned char* p, bool fast, int nv) {
+  if (fast) {
+    r[0] = (int)ldg1(p);
+  } else {
+    unsigned c = 0;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) c |= (i < nv ? (unsigned)__ldg(p + i) : 0u) << (8 * i);
+    r[0] = (int)c;
+  }
+}
+// Row i of the fetched words.
+WS_DI unsigned code4(const int (&r)[1], int i) { return ((unsigned)r[0] >> (8 * i)) & 0xffu; }
+WS_DI unsigned code4(const int (&r)[2], int i) { return ((unsigned)r[i >> 1] >> (16 * (i & 1))) & 0xffffu; }
+WS_DI unsigned code4(const int (&r)[4], int i) { return (unsigned)r[i]; }
+WS_DI i64 word4(const int (&r)[8], int i) { return (i64)(((u64)(unsigned)r[2 * i + 1] << 32) | (unsigned)r[2 * i]); }
+
+// a / b for b with the correctly rounded reciprocal y (0: not prepared, divide): the quotient estimate
+// a y is corrected twice by its exact remainder, after the first of which it is within one unit in the last
+// place, so the second gives the correctly rounded quotient (Markstein, "Computation of elementary functions
+// on the IBM RISC System/6000 processor", 1990, theorem on correctly rounded quotients).  Used with integers
+// below 2^52 and b = 10^s, where nothing overflows or underflows.  Five multiply-adds instead of the
+// division's sequence, which the compiler repeats for each of the four rows.
+WS_DI double quotRecip(double a, double b, double y) {
+  if (y == 0.0) return a / b;
+  double q = a * y;
+  q = fma(fma(-q, b, a), y, q);
+  return fma(fma(-q, b, a), y, q);
+}
+// The reciprocal quotRecip takes for a decimal column with this base and divisor, or 0.
+WS_DI double quotPrepare(i64 base, double b) {
+  const i64 lim = 1ll << 51;
+  return base > -lim && base < lim && b >= 1.0 && b <= 1e15 ? 1.0 / b : 0.0;
 }
 
 // Four consecutive rows of a column.  `fast`: the group is full and its address is aligned to
@@ -637,6 +713,8 @@ struct Launch {
   int stages;                 // shared-memory stages of staged scans (0: loads straight from global memory)
   int sumShift;               // integer SUM words need no overflow test while (argument magnitude >> sumShift)
                               // is 0 (set at launch from the rows a thread adds; -1: always test)
+  int copies;                 // dense GROUP BY in shared memory: copies of each group (a power of two)
+  int kmin32;                 // dense GROUP BY: every |kmin| <= 2^30 (32-bit key arithmetic is exact, see denseIndex)
   int waitLog2;               // staged scans: a wait for a tile stage gives up after 2^waitLog2 SM cycles
   // A launch serving several queries gives each its own range of CTAs: this query's first CTA and its
   // CTA count (0: the whole grid).  Bodies use ctaIndex / ctaCount, never blockIdx / gridDim.
@@ -659,8 +737,8 @@ struct Launch {
   int spillRows;              // per-CTA shared buffer of rows bound for the global table (hash GROUP BY)
   int probeLimit;             // global probe limit before reporting overflow
   // selection
-  i64* tileCount;             // [ntiles] selected rows per tile (count pass) / exclusive offsets (write pass)
-  int32_t* outIdx;
+  i64* tileCount;             // [ntiles] selected rows per tile
+  uint32_t* selMask;          // [ntiles * kTile / 32] a bit per row
 };
 
 WS_DI unsigned ctaIndex(const Launch& L) { return blockIdx.x - (unsigned)L.ctaBase; }

@@ -53,6 +53,7 @@ int smCount();
 int arch();
 cudaStream_t stream();           // the calling thread's stream (ws_set_stream), default per-thread
 void* tmpAlloc(size_t bytes);    // stream-ordered pool allocation on stream()
+void* tableAlloc(size_t bytes);  // the same for result tables: large ones from a pool of their own (freed by tmpFree)
 void tmpFree(void* p);
 void h2dAsync(void* d, const void* h, size_t b);
 void d2hSync(void* h, const void* d, size_t b);
@@ -85,6 +86,7 @@ struct DBuf {
   int64_t n = 0;
   DBuf() = default;
   explicit DBuf(int64_t count) : n(count) { p = count > 0 ? (T*)tmpAlloc(sizeof(T) * count) : nullptr; }
+  DBuf(T* own, int64_t count) : p(own), n(count) {}  // takes a pool allocation over
   DBuf(const DBuf&) = delete;
   DBuf& operator=(const DBuf&) = delete;
   DBuf(DBuf&& o) noexcept : p(o.p), n(o.n) { o.p = nullptr, o.n = 0; }
@@ -146,13 +148,14 @@ EnvK envK(const ws_expr_env& env);
 // ---------------------------------------------------------------- kernels
 // The scan kernels of one evaluator: the interpreter's (built into the library) or a compiled plan's.
 // K_DENSE_PRIV: direct loads, kThreads threads, bounded for several resident CTAs per SM;
-// K_DENSE_PRIV_STAGED: the same body with a producer warp staging tiles by TMA (kStagedThreads).
+// K_DENSE_PRIV_STAGED, K_NOKEYS_STAGED: the same bodies with a producer warp staging tiles by TMA (kStagedThreads).
 enum KernelId {
-  K_NOKEYS = 0, K_DENSE_SHARED, K_DENSE_GLOBAL, K_HASH, K_SELECT_COUNT, K_SELECT_WRITE, K_DENSE_PRIV,
-  K_DENSE_PRIV_STAGED, K_MULTI_NOKEYS, K_MULTI_DENSE_PRIV, K_MULTI_HASH, K_COUNT_
+  K_NOKEYS = 0, K_DENSE_SHARED, K_DENSE_GLOBAL, K_HASH, K_SELECT, K_DENSE_PRIV,
+  K_DENSE_PRIV_STAGED, K_MULTI_NOKEYS, K_MULTI_DENSE_PRIV, K_MULTI_HASH, K_NOKEYS_STAGED, K_COUNT_
 };
 struct KernelSet {
   CUfunction fn[K_COUNT_] = {};
+  int denseV = 1;  // K_DENSE_SHARED's CTA: denseV * kThreads threads
   bool interp = true;
 };
 const KernelSet& interpKernels();
@@ -175,11 +178,24 @@ struct ws_jit_program {
   int id = 0;
   int fnKind = 0;
   std::string kind, sql, source;
+  std::string kernelSource;  // kernel instantiations compiled after `source`
+  // hot: `kernels` are instantiated with the evaluator of hinted storage, which only runs batches whose columns
+  // are stored as `encs` (column, encoding) says; `generic` runs any batch the plan covers.
+  bool hot = false;
+  std::vector<std::pair<int, int>> encs;
   double compileMs = 0;
   std::atomic<int> state{0};  // 0 compiling, 1 ready, 2 failed
   bool fromDisk = false;
   int stageBytes = 0;  // shared memory per staged tile (0: the plan reads global memory directly)
-  ws::KernelSet kernels;
+  ws::KernelSet kernels, generic;
+  // The kernels that can run these batches.
+  const ws::KernelSet& kernelsFor(int nb, int ncols, const ws_col_view* bcols) const {
+    if (!hot) return kernels;
+    for (int b = 0; b < nb; ++b)
+      for (auto& [c, e] : encs)
+        if (bcols[(int64_t)b * ncols + c].enc != e) return generic;
+    return kernels;
+  }
   CUmodule module = nullptr;
   std::mutex mu;
   int64_t execs = 0;

@@ -4,11 +4,16 @@
 //
 // Evaluator contract (all row indices are within the current batch):
 //   static constexpr int NK, NA;            loop bounds (>= nk(), na())
+//   static constexpr bool COMPACT;          shared tables hold compact accumulators (else accumulator rows)
+//   static constexpr int DENSE_V, FLUSH_ROWS, *_MIN_BLOCKS;   see the kernels
 //   Ev(const Launch&);  void bind(const Launch&, int batch);  bool fastOk;
 //   int nk(), na(), rowWords(), kind(a), woff(a); bool keyInt(k);
 //   void load(i64 r0, bool fast, int nv);   rows r0 .. r0+3 (nv valid) into registers
 //   bool where(i); i64 ikey(k, i); double dkey(k, i); bool ival(a, i, i64&); double dval(a, i)
 //   void prep(i, bool live); void finish()
+// Evaluators with HOT = true (columns of known storage) keep the fetched rows packed and decode a row where it
+// is used; they evaluate only rows that passed (prep), and give sumMag(i), the magnitude word of row i's SUM
+// arguments (see sumMagnitude), and for the GROUP BY keys of KEY32 (a bit per key) ikey32(k, i).
 //
 // Work decomposition: a batch (segment / write buffer) is cut into tiles of kTile rows; a CTA of
 // kThreads threads takes one tile per iteration, each thread 4 consecutive rows (128-bit loads of
@@ -41,8 +46,15 @@ WS_DI void rowGroup(Ev& ev, unsigned live, int b, i64 r0, F&& f) {
 #pragma unroll
   for (int i = 0; i < 4; ++i) {
     const bool ok = ((live >> i) & 1u) && ev.where(i);
-    ev.prep(i, ok);
-    if (ok) f(i, b, r0 + i);
+    if constexpr (Ev::HOT) {
+      if (ok) {
+        ev.prep(i, true);
+        f(i, b, r0 + i);
+      }
+    } else {
+      ev.prep(i, ok);
+      if (ok) f(i, b, r0 + i);
+    }
   }
 }
 
@@ -63,9 +75,12 @@ WS_DI int batchOfTile(const Launch& L, i64 t) {
 // rather than once per batch of the launch.  tile(t, b, r0, n, del) is called by every thread of the
 // CTA for each tile t of batch b (r0 = the thread's first row in the batch, n = the batch's rows,
 // del = its deleted bitmap); it returns true to end the walk (the same value in every thread).
-template <class Ev, class F>
+// V > 1: a CTA of V * kThreads threads walks as V CTAs of kThreads would (V ranges, one per group of kThreads
+// threads); its body then has no CTA-wide barrier in the walk.
+template <int V = 1, class Ev, class F>
 WS_DI void forEachOwnedTile(const Launch& L, Ev& ev, F&& tile) {
-  const i64 T = L.ntiles, G = ctaCount(L), c = ctaIndex(L);
+  const i64 T = L.ntiles, G = (i64)ctaCount(L) * V, c = (i64)ctaIndex(L) * V + (V > 1 ? threadIdx.x / kThreads : 0);
+  const int tid = V > 1 ? threadIdx.x % kThreads : threadIdx.x;
   i64 t = T * c / G;
   const i64 tEnd = T * (c + 1) / G;
   if (t >= tEnd) return;
@@ -76,7 +91,7 @@ WS_DI void forEachOwnedTile(const Launch& L, Ev& ev, F&& tile) {
     const i64 n = __ldg(L.n + b);
     const uint32_t* del = L.del[b];
     for (; t < be; ++t)
-      if (tile(t, b, (t - bs) * kTile + threadIdx.x * 4, n, del)) return;
+      if (tile(t, b, (t - bs) * kTile + tid * 4, n, del)) return;
   }
 }
 
@@ -105,9 +120,9 @@ WS_DI void forEachRowTiles(const Launch& L, Ev& ev, F&& f, E&& tileEnd) {
   ev.finish();
 }
 
-template <class Ev, class F>
+template <int V = 1, class Ev, class F>
 WS_DI void forEachRow(const Launch& L, Ev& ev, F&& f) {
-  forEachOwnedTile(L, ev, [&](i64, int b, i64 r0, i64 n, const uint32_t* del) {
+  forEachOwnedTile<V>(L, ev, [&](i64, int b, i64 r0, i64 n, const uint32_t* del) {
     visitRows(ev, b, r0, n, del, f);
     return false;
   });
@@ -294,7 +309,8 @@ WS_DI void addCarry(u64* w, u64 x, u64* spillHi) {
 // additions (signed overflow carried into the int128 spill) for the rest of the launch, so words that
 // take unbounded values are always tested from their first such value on.
 template <class Ev>
-WS_DI unsigned sumMagnitude(const Ev& ev, const u64* x) {
+WS_DI unsigned sumMagnitude(const Ev& ev, const u64* x, int i) {
+  if constexpr (Ev::HOT) return ev.sumMag(i);
   unsigned m = 0;
 #pragma unroll
   for (int a = 0; a < Ev::NA; ++a) {
@@ -488,11 +504,55 @@ WS_DI void blockReduceRow(const Ev& ev, u64 (&w)[RW], u64* sred /* [kStagedThrea
   __syncthreads();
 }
 
+// (lo, hi) += (l, h) for one slot of kind k.
+WS_DI void slotIdentity(int k, u64& lo, u64& hi) {
+  hi = 0;
+  lo = k == SK_IMIN ? (u64)0x7fffffffffffffffll : k == SK_IMAX ? (u64)0x8000000000000000ll
+       : k == SK_DMIN ? (u64)dord(__longlong_as_double(0x7ff0000000000000ll))
+       : k == SK_DMAX ? (u64)dord(__longlong_as_double((i64)0xfff0000000000000ull)) : 0ull;
+}
+WS_DI void slotCombine(int k, u64& lo, u64& hi, u64 l, u64 h) {
+  switch (k) {
+    case SK_COUNT: lo += l; break;
+    case SK_ISUM: add128w(lo, *(i64*)&hi, l, (i64)h); break;
+    case SK_IMIN: case SK_DMIN: if ((i64)l < (i64)lo) lo = l; break;
+    case SK_IMAX: case SK_DMAX: if ((i64)l > (i64)lo) lo = l; break;
+    case SK_DSUM: lo = (u64)__double_as_longlong(__longlong_as_double((i64)lo) + __longlong_as_double((i64)l)); break;
+    default: break;
+  }
+}
+// Reduces every (row, slot) of nrows rows over N contributors, one pair per warp at a time: lane l folds
+// contributors l, l + 32, ... in order, then a fixed shuffle tree combines the lanes (deterministic), and lane 0
+// calls put(row, slot, lo, hi).  get(row, slot, contributor, lo, hi) reads a value.  A pair moves its one or two
+// words only and needs no barrier, where whole rows went through every shuffle group by group.
+template <class Ev, class Get, class Put>
+WS_DI void reducePairs(const Ev& ev, int nrows, int N, Get&& get, Put&& put) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5, na = ev.na();
+  for (int p = warp; p < nrows * na; p += nw) {
+    const int r = p / na, a = p % na, k = ev.kind(a);
+    if (k == SK_NONE) continue;
+    u64 lo, hi;
+    slotIdentity(k, lo, hi);
+#pragma unroll 4
+    for (int c = lane; c < N; c += 32) {
+      u64 l, h;
+      get(r, a, c, l, h);
+      slotCombine(k, lo, hi, l, h);
+    }
+#pragma unroll
+    for (int off = 16; off > 0; off >>= 1) {
+      const u64 l = __shfl_down_sync(0xffffffffu, lo, off), h = __shfl_down_sync(0xffffffffu, hi, off);
+      slotCombine(k, lo, hi, l, h);
+    }
+    if (lane == 0) put(r, a, lo, hi);
+  }
+}
+
 // After every CTA wrote its partial rows part[cta][nrows][rw]: the last CTA to finish reduces them
-// into rows[nrows][rw] (word 0 of each row = its key word, left as is).  Thread t folds CTAs t,
-// t + blockDim, ... in order, then a fixed-shape tree combines the threads: deterministic.
-template <class Ev, int RW>
-WS_DI void lastCtaReduce(const Launch& L, const Ev& ev, int nrows, u64* sred) {
+// into rows[nrows][rw] (word 0 of each row = its key word, left as is; rows accumulate across launches (scan
+// windows): combined into them), deterministically.
+template <class Ev>
+WS_DI void lastCtaReduce(const Launch& L, const Ev& ev, int nrows) {
   __shared__ bool amLast;
   __threadfence();
   __syncthreads();
@@ -501,32 +561,25 @@ WS_DI void lastCtaReduce(const Launch& L, const Ev& ev, int nrows, u64* sred) {
   if (!amLast) return;
   __threadfence();
   const int rw = ev.rowWords();
-  for (int g = 0; g < nrows; ++g) {
-    u64 w[RW];
-    rowIdentity(ev, w);
-    for (unsigned c = threadIdx.x; c < ctaCount(L); c += blockDim.x) {
-      const u64* p = L.part + ((size_t)c * nrows + g) * rw;
-      u64 x[RW];
-#pragma unroll
-      for (int j = 1; j < RW; ++j) x[j] = j < rw ? __ldcg(p + j) : 0;
-      rowCombine(ev, w, x);
-    }
-    blockReduceRow(ev, w, sred);
-    if (threadIdx.x == 0) {  // rows accumulate across launches (scan windows): combine into them
-      u64* out = L.rows + (size_t)g * rw;
-      u64 x[RW];
-#pragma unroll
-      for (int j = 1; j < RW; ++j) x[j] = j < rw ? out[j] : 0;
-      rowCombine(ev, x, w);
-#pragma unroll
-      for (int j = 1; j < RW; ++j)
-        if (j < rw) out[j] = x[j];
-    }
-  }
+  reducePairs(
+      ev, nrows, (int)ctaCount(L),
+      [&](int r, int a, int c, u64& lo, u64& hi) {
+        const u64* p = L.part + ((size_t)c * nrows + r) * rw + ev.woff(a);
+        lo = __ldcg(p);
+        hi = ev.kind(a) == SK_ISUM ? __ldcg(p + 1) : 0ull;
+      },
+      [&](int r, int a, u64 lo, u64 hi) {
+        u64* out = L.rows + (size_t)r * rw + ev.woff(a);
+        const bool two = ev.kind(a) == SK_ISUM;
+        u64 l = out[0], h = two ? out[1] : 0ull;
+        slotCombine(ev.kind(a), l, h, lo, hi);
+        out[0] = l;
+        if (two) out[1] = h;
+      });
 }
 
 // ------------------------------------------------------------------ no GROUP BY
-template <class Ev>
+template <class Ev, bool kStaged>
 __device__ void aggNoKeys(const Launch& L) {
   constexpr int RW = Ev::RW, FW = Ev::FRW;
   __shared__ u64 sred[(kStagedThreads / 32) * RW];
@@ -536,13 +589,33 @@ __device__ void aggNoKeys(const Launch& L) {
   __syncthreads();
   u64 f[FW];
   fastIdentity(ev, f);
-  // register rows: a tested addition costs about what the magnitude test of the bounded form does
-  // (no shared-memory ordering is at stake), so every addition is tested here
-  scanRows(L, ev, [&](int i, int, i64) {
+  bool tested = false;  // sums take tested additions (sticky, see sumMagnitude)
+  // A HOT evaluator knows most rows' magnitudes from its narrow evaluation, so the bounded form pays; for the
+  // others a tested addition costs about what the magnitude test does, so every addition is tested.
+  auto row = [&](int i, int, i64) {
     u64 x[FW];
     fastOfInput(ev, i, x);
+    if constexpr (Ev::HOT) {
+      tested |= sumsNeedTests(L, ev.sumMag(i));
+      if (!tested) {
+#pragma unroll
+        for (int a = 0; a < Ev::NA; ++a) {
+          const int o = ev.fwoff(a);
+          switch (ev.kind(a)) {
+            case SK_COUNT: case SK_ISUM: f[o] += x[o]; break;
+            case SK_IMIN: case SK_DMIN: if ((i64)x[o] < (i64)f[o]) f[o] = x[o]; break;
+            case SK_IMAX: case SK_DMAX: if ((i64)x[o] > (i64)f[o]) f[o] = x[o]; break;
+            case SK_DSUM: f[o] = (u64)__double_as_longlong(__longlong_as_double((i64)f[o]) + __longlong_as_double((i64)x[o])); break;
+            default: break;
+          }
+        }
+        return;
+      }
+    }
     fastCombine(ev, f, x, spill);
-  });
+  };
+  if constexpr (kStaged) scanRows(L, ev, row);
+  else forEachRow(L, ev, row);
   u64 w[RW];
   rowIdentity(ev, w);
   fastExpand(ev, f, w);
@@ -554,7 +627,7 @@ __device__ void aggNoKeys(const Launch& L) {
       if (ev.kind(a) == SK_ISUM) add128w(w[ev.woff(a)], *(i64*)&w[ev.woff(a) + 1], spill[2 * a], (i64)spill[2 * a + 1]);
     for (int j = 1; j < rw; ++j) L.part[(size_t)ctaIndex(L) * rw + j] = w[j];
   }
-  lastCtaReduce<Ev, RW>(L, ev, 1, sred);
+  lastCtaReduce(L, ev, 1);
 }
 
 // ------------------------------------------------------------------ dense GROUP BY
@@ -562,6 +635,27 @@ template <class Ev>
 WS_DI bool denseIndex(const Launch& L, const Ev& ev, int i, i64& g) {
   // ranges and G are below 2^26 (the dense limit), so the index arithmetic fits 32 bits
   unsigned gg = 0;
+  if constexpr (Ev::HOT && Ev::KEY32 != 0) {
+    // int32 keys with |kmin| <= 2^30: key - kmin lies in [-3 * 2^30, 3 * 2^30), so a negative difference's low
+    // word is at least 2^30 and only differences in the range (< 2^26) are below it
+    if (L.kmin32) {
+#pragma unroll
+      for (int k = 0; k < Ev::NK; ++k) {
+        if (k >= ev.nk()) break;
+        unsigned d;
+        if ((Ev::KEY32 >> k) & 1) {
+          d = (unsigned)ev.ikey32(k, i) - (unsigned)(int)L.kmin[k];
+        } else {
+          const i64 dd = ev.ikey(k, i) - L.kmin[k];
+          d = (u64)dd >> 32 ? 0xffffffffu : (unsigned)dd;
+        }
+        if (d >= (unsigned)L.range[k]) return false;
+        gg += d * (unsigned)L.stride[k];
+      }
+      g = gg;
+      return gg < (unsigned)L.G;
+    }
+  }
 #pragma unroll
   for (int k = 0; k < Ev::NK; ++k) {
     if (k >= ev.nk()) break;
@@ -581,9 +675,8 @@ WS_DI bool denseIndex(const Launch& L, const Ev& ev, int i, i64& g) {
 // the last CTA reduces them.
 template <class Ev, bool kStaged>
 __device__ void aggDensePriv(const Launch& L) {
-  constexpr int RW = Ev::RW, FW = Ev::FRW, T = kThreads;
+  constexpr int FW = Ev::FRW, T = kThreads;
   extern __shared__ __align__(16) u64 wsSmem[];
-  __shared__ u64 sred[(kStagedThreads / 32) * RW];
   Ev ev(L);
   const int G = (int)L.G, tid = threadIdx.x;
   const bool owner = tid < T;  // the producer warp of a staged launch owns no rows
@@ -608,7 +701,7 @@ __device__ void aggDensePriv(const Launch& L) {
     }
     u64 x[FW];
     fastOfInput(ev, i, x);
-    tested |= sumsNeedTests(L, sumMagnitude(ev, x));
+    tested |= sumsNeedTests(L, sumMagnitude(ev, x, i));
     u64* p = priv + ((unsigned)gi * (unsigned)fw * T + tid);
     if (!tested) {  // no atomics on this path: the slots' read-modify-writes overlap
 #pragma unroll
@@ -647,38 +740,175 @@ __device__ void aggDensePriv(const Launch& L) {
   else forEachRow(L, ev, row);
   __syncthreads();
   const int rw = ev.rowWords();
-  for (int g = 0; g < G; ++g) {
-    u64 f[FW];
-    fastIdentity(ev, f);
-    if (owner)
-#pragma unroll
-      for (int j = 0; j < FW; ++j)
-        if (j < fw) f[j] = priv[((size_t)g * fw + j) * T + tid];
-    u64 w[RW];
-    rowIdentity(ev, w);
-    fastExpand(ev, f, w);
-    blockReduceRow(ev, w, sred);
-    if (tid == 0) {
-      const u64* sp = spill + (size_t)g * 2 * Ev::NA;
-      for (int a = 0; a < ev.na(); ++a)
-        if (ev.kind(a) == SK_ISUM) add128w(w[ev.woff(a)], *(i64*)&w[ev.woff(a) + 1], sp[2 * a], (i64)sp[2 * a + 1]);
-      for (int j = 1; j < rw; ++j) L.part[((size_t)ctaIndex(L) * G + g) * rw + j] = w[j];
-    }
-  }
-  lastCtaReduce<Ev, RW>(L, ev, G, sred);
+  reducePairs(
+      ev, G, T,
+      [&](int g, int a, int c, u64& lo, u64& hi) {
+        lo = priv[((size_t)g * fw + ev.fwoff(a)) * T + c];
+        hi = ev.kind(a) == SK_ISUM ? (u64)((i64)lo >> 63) : 0ull;
+      },
+      [&](int g, int a, u64 lo, u64 hi) {
+        const u64* sp = spill + ((size_t)g * Ev::NA + a) * 2;
+        u64* out = L.part + ((size_t)ctaIndex(L) * G + g) * rw + ev.woff(a);
+        if (ev.kind(a) == SK_ISUM) {
+          add128w(lo, *(i64*)&hi, sp[0], (i64)sp[1]);
+          out[1] = hi;
+        }
+        out[0] = lo;
+      });
+  lastCtaReduce(L, ev, G);
 }
 
-// Medium G: the CTA's rows [G][rw] live in shared memory (rows' key words unused) and take shared
-// atomics; at the end each non-empty group is merged into the global rows with global atomics.
+// ------------------------------------------------------------------ compact accumulators
+// A group's accumulators in a CTA's shared-memory table: a 64-bit word per slot (COUNT: 32 bits, in an array of
+// their own), updated by 32-bit shared atomics where a 64-bit one would be a compare-and-swap loop:
+//   COUNT   one 32-bit addition (a CTA visits fewer than 2^32 rows);
+//   integer SUM   the low half added with its old value returned, the high half and the carry only when that sum
+//           is not zero, i.e. rarely for small non-negative arguments.  The word is exact modulo 2^64 and must not leave the
+//           int64 range: a row whose arguments break the bound of sumMagnitude for the whole CTA's rows
+//           (compactOk) does not go through the table;
+//   MIN / MAX   a read, and an atomic only when the row improves on it;
+//   DOUBLE SUM   a 64-bit atomic.
+// A table of E entries holds each slot's words together (word o64 of entry e at t64[o64 * E + e]): the lanes of a warp
+// update one slot of random entries at a time, which then spread over all banks (words entry by entry, four to an
+// entry, met in 4 bank pairs, 98 shared-memory wavefronts per 32 rows of five aggregates: 168 us where this takes 118).
+// Against accumulator rows of 64-bit and 128-bit words: 36 instead of 56 bytes for COUNT, SUM, MIN, MAX and a DOUBLE
+// SUM, so the table takes more groups or leaves room for more warps.
+//
+// The interpreter (COMPACT = false) keeps whole accumulator rows there, entry by entry: its slots' kinds and offsets are
+// not constants, and the branches above cost it more than the atomics (1500 groups, 4M rows: 0.87 ms with rows, 5 to
+// 13 ms with compact words, depending on the unrolling).
+//
+// t64 / t32: the table's words, E entries; e: an entry; x: a row's accumulator words (rowOfInput).
+template <class Ev>
+WS_DI void compactWords(const Ev& ev, int& n64, int& n32) {
+  n64 = n32 = 0;
+  if constexpr (!Ev::COMPACT) {
+    n64 = ev.rowWords();
+  } else {
+#pragma unroll
+    for (int a = 0; a < Ev::NA; ++a) {
+      const int k = ev.kind(a);
+      n32 += k == SK_COUNT;
+      n64 += k != SK_COUNT && k != SK_NONE;
+    }
+  }
+}
+template <class Ev>
+WS_DI void compactIdentity(const Ev& ev, u64* t64, unsigned* t32, unsigned e, unsigned E) {
+  if constexpr (!Ev::COMPACT) {
+    rowIdentity(ev, t64 + (size_t)e * ev.rowWords());
+  } else {
+    unsigned o64 = e, o32 = e;
+#pragma unroll
+    for (int a = 0; a < Ev::NA; ++a) {
+      const int k = ev.kind(a);
+      if (k == SK_NONE) continue;
+      if (k == SK_COUNT) {
+        t32[o32] = 0, o32 += E;
+      } else {
+        u64 hi;
+        slotIdentity(k, t64[o64], hi);
+        o64 += E;
+      }
+    }
+  }
+}
+// Row i (words x) may be added to compact words: the sums of all the CTA's rows (2^8 threads of at most
+// 2^(31 - sumShift) rows each) stay in the int64 range.
+template <class Ev>
+WS_DI bool compactOk(const Launch& L, const Ev& ev, const u64* x, int i) {
+  if constexpr (!Ev::COMPACT) return true;
+  unsigned m = 0;
+  if constexpr (Ev::HOT) {
+    m = ev.sumMag(i);
+  } else {
+#pragma unroll
+    for (int a = 0; a < Ev::NA; ++a)
+      if (ev.kind(a) == SK_ISUM) m |= magHigh((i64)x[ev.woff(a)]);
+  }
+  return L.sumShift >= 8 && (m >> (L.sumShift - 8)) == 0;
+}
+template <class Ev>
+WS_DI void compactAdd(const Ev& ev, const u64* x, u64* t64, unsigned* t32, unsigned e, unsigned E) {
+  if constexpr (!Ev::COMPACT) {
+    rowAtomicCombine(ev, t64 + (size_t)e * ev.rowWords(), x);
+  } else {
+    unsigned o64 = e, o32 = e;
+#pragma unroll
+    for (int a = 0; a < Ev::NA; ++a) {
+      const int k = ev.kind(a);
+      if (k == SK_NONE) continue;
+      const u64 v = x[ev.woff(a)];
+      if (k == SK_COUNT) {
+        atomicAdd(t32 + o32, 1u);
+        o32 += E;
+        continue;
+      }
+      u64* p = t64 + o64;
+      o64 += E;
+      switch (k) {
+        case SK_ISUM: {
+          const unsigned lo = (unsigned)v;
+          unsigned h = (unsigned)(v >> 32);
+          if (lo) h += atomicAdd((unsigned*)p, lo) + lo < lo;  // the carry of the low half
+          if (h) atomicAdd((unsigned*)p + 1, h);
+          break;
+        }
+        case SK_IMIN: case SK_DMIN: if ((i64)v < *(volatile i64*)p) atomicMin((i64*)p, (i64)v); break;
+        case SK_IMAX: case SK_DMAX: if ((i64)v > *(volatile i64*)p) atomicMax((i64*)p, (i64)v); break;
+        case SK_DSUM: {
+          const double d = __longlong_as_double((i64)v);
+          if (d != 0.0) atomicAdd((double*)p, d);
+          break;
+        }
+        default: break;
+      }
+    }
+  }
+}
+// w (an accumulator row) += entry e
+template <class Ev>
+WS_DI void compactInto(const Ev& ev, u64* w, const u64* t64, const unsigned* t32, unsigned e, unsigned E) {
+  if constexpr (!Ev::COMPACT) {
+    rowCombine(ev, w, t64 + (size_t)e * ev.rowWords());
+  } else {
+    unsigned o64 = e, o32 = e;
+#pragma unroll
+    for (int a = 0; a < Ev::NA; ++a) {
+      const int k = ev.kind(a), o = ev.woff(a);
+      if (k == SK_NONE) continue;
+      if (k == SK_COUNT) {
+        w[o] += t32[o32], o32 += E;
+      } else {
+        const u64 v = t64[o64];
+        o64 += E;
+        u64 one = 0;
+        slotCombine(k, w[o], k == SK_ISUM ? w[o + 1] : one, v, (u64)((i64)v >> 63));
+      }
+    }
+  }
+}
+
+// Medium G: the CTA's groups live in shared memory as compact accumulators, L.copies of each (a power of two; a
+// lane uses copy lane % copies, which spreads the lanes of a warp that meet in one of few groups); at the end
+// each non-empty group is merged into the global rows with global atomics.  One CTA of Ev::DENSE_V * kThreads
+// threads shares a table, so that an SM holds the warps of several CTAs but merges one or two tables: 16.8M
+// rows into 1500 groups with five aggregates 215 -> 118 us (accumulator rows of 56 B and CTAs of 256 threads left 16
+// warps per SM), 12M into 5000 groups 377 -> 83 us (those rows did not fit, every row went to L2 atomics).  What bounds
+// it now is the shared-memory pipe (88 % busy): the atomics of random entries.
 template <class Ev>
 __device__ void aggDenseShared(const Launch& L) {
   extern __shared__ __align__(16) u64 wsSmem[];
   Ev ev(L);
-  const int rw = ev.rowWords();
-  const i64 G = L.G;
-  for (i64 g = threadIdx.x; g < G; g += blockDim.x) rowIdentity(ev, wsSmem + g * rw);
+  const int rw = ev.rowWords(), G = (int)L.G, C = L.copies, E = G * C;
+  int n64, n32;
+  compactWords(ev, n64, n32);
+  u64* t64 = wsSmem;
+  unsigned* t32 = (unsigned*)(t64 + (size_t)E * n64);
+  for (int e = threadIdx.x; e < E; e += blockDim.x) compactIdentity(ev, t64, t32, e, E);
   __syncthreads();
-  forEachRow(L, ev, [&](int i, int, i64) {
+  const int copy = threadIdx.x & (C - 1);
+  forEachRow<Ev::DENSE_V>(L, ev, [&](int i, int, i64) {
     i64 gi;
     if (!denseIndex(L, ev, i, gi)) {
       L.err[0] = 1;
@@ -686,13 +916,20 @@ __device__ void aggDenseShared(const Launch& L) {
     }
     u64 x[kMaxRowWords];
     rowOfInput(ev, i, x);
-    rowAtomicCombine(ev, wsSmem + gi * rw, x);
+    if (compactOk(L, ev, x, i)) {
+      const int e = (int)gi * C + copy;
+      compactAdd(ev, x, t64, t32, e, E);
+    } else {
+      rowAtomicCombine(ev, L.rows + gi * rw, x);
+    }
   });
   __syncthreads();
-  for (i64 g = threadIdx.x; g < G; g += blockDim.x) {
-    const u64* s = wsSmem + g * rw;
-    if (s[ev.woff(0)] == 0) continue;  // slot 0 is COUNT(*): no rows of this group in this CTA
-    rowAtomicCombine(ev, L.rows + g * rw, s);
+  for (int g = threadIdx.x; g < G; g += blockDim.x) {
+    u64 w[kMaxRowWords];
+    rowIdentity(ev, w);
+    for (int c = 0; c < C; ++c) compactInto(ev, w, t64, t32, g * C + c, E);
+    if (w[ev.woff(0)] == 0) continue;  // slot 0 is COUNT(*): no rows of this group in this CTA
+    rowAtomicCombine(ev, L.rows + (i64)g * rw, w);
   }
 }
 
@@ -735,14 +972,18 @@ WS_DI u64 keyWord(const Ev& ev, int i, double* kv) {
   return h == kEmpty ? (h ^ 1) : h;
 }
 
-// Inserts accumulator row x under key word kw into the global table (linear probing, bounded).
+// The key word in key word kw's first slot of the global table, as last seen (globalInsert's starting point).
 template <class Ev>
-WS_DI void globalInsert(const Launch& L, const Ev& ev, u64 kw, const double* kv, const u64* x) {
-  if (*(volatile int*)(L.err + 1)) return;  // the table overflowed: the caller reruns with a bigger one
+WS_DI u64 globalPeek(const Launch& L, const Ev& ev, u64 kw) {
+  return *(volatile u64*)(L.table + (mix64(kw) & L.mask) * ev.rowWords());
+}
+// Inserts accumulator row x under key word kw into the global table (linear probing, bounded); first: globalPeek.
+template <class Ev>
+WS_DI void globalInsert(const Launch& L, const Ev& ev, u64 kw, const double* kv, const u64* x, u64 first) {
   const int rw = ev.rowWords();
-  if (kw == kEmpty) {  // the EMPTY key word itself has a dedicated row after the table
+  if (kw == kEmpty) {  // the EMPTY key word itself has a dedicated row after the table (a single key: it is the key)
     u64* row = L.table + (L.mask + 1) * rw;
-    if (atomicCAS(row, 0ull, 1ull) == 0ull)
+    if (atomicCAS(row, 0ull, 1ull) == 0ull && ev.nk() > 1)
       for (int k = 0; k < ev.nk(); ++k) L.tkeys[(L.mask + 1) * ev.nk() + k] = kv[k];
     rowAtomicCombine(ev, row, x);
     return;
@@ -750,7 +991,7 @@ WS_DI void globalInsert(const Launch& L, const Ev& ev, u64 kw, const double* kv,
   u64 s = mix64(kw) & L.mask;
   for (int p = 0; p < L.probeLimit; ++p) {
     u64* row = L.table + s * rw;
-    u64 prev = *(volatile u64*)row;
+    u64 prev = p ? *(volatile u64*)row : first;
     if (prev == kEmpty) {
       prev = atomicCAS(row, kEmpty, kw);
       if (prev == kEmpty) {
@@ -770,54 +1011,95 @@ WS_DI void globalInsert(const Launch& L, const Ev& ev, u64 kw, const double* kv,
   L.err[1] = 1;  // no free slot within the probe limit
 }
 
-// Rows are pre-aggregated in a per-CTA shared-memory table (smemSlots rows, bounded probing), which
-// absorbs hot keys.  A row that finds no slot there is appended to a per-CTA shared buffer (one
-// shared atomic per warp); after each tile the whole CTA inserts the buffered rows into the global
-// table together, one row per thread, so the global probes and atomics of the cold keys run with all
-// lanes active instead of a few diverged lanes at a time.  (A row finding the buffer full goes to
-// the global table directly.)  The shared table is merged into the global table when the CTA finishes.
-// Shared memory: [S][rw] table | [S][nk] key values (multi-key) | [B][rw] buffer | [B][nk] key values.
+// A list of n rows into the global table, Ev::FLUSH_ROWS per thread at a time: key(j) is row j's key word (kEmpty:
+// no first probe), insert(j, key word, first) inserts it.
+template <class Ev, class Key, class Insert>
+WS_DI void insertAll(const Launch& L, const Ev& ev, int n, Key&& key, Insert&& insert) {
+  for (int j0 = threadIdx.x; j0 < n; j0 += blockDim.x * Ev::FLUSH_ROWS) {
+    u64 kw[Ev::FLUSH_ROWS], first[Ev::FLUSH_ROWS];
+#pragma unroll
+    for (int r = 0; r < Ev::FLUSH_ROWS; ++r) {
+      const int j = j0 + r * (int)blockDim.x;
+      kw[r] = j < n ? key(j) : kEmpty;
+      first[r] = kw[r] != kEmpty ? globalPeek(L, ev, kw[r]) : 0ull;
+    }
+#pragma unroll
+    for (int r = 0; r < Ev::FLUSH_ROWS; ++r) {
+      const int j = j0 + r * (int)blockDim.x;
+      if (j < n) insert(j, kw[r], first[r]);
+    }
+  }
+}
+
+// Rows are pre-aggregated in a per-CTA shared-memory table (smemSlots key words with compact accumulators,
+// bounded probing), which absorbs hot keys.  A row that finds no slot there (or whose sums exceed the compact
+// bound) is appended to a per-CTA shared buffer (one shared atomic per warp); after a tile that appended any, the
+// whole CTA inserts the buffered rows into the global table together, Ev::FLUSH_ROWS rows per
+// thread at a time whose first probes are all in flight before the first is waited for, so the global probes and
+// atomics of the cold keys run with all lanes active and overlap.  (A row finding the buffer full goes to the
+// global table directly.)  The shared table is merged into the global table when the CTA finishes.
+// A tile without such rows costs one CTA barrier, which also votes on the flush: a thread knows whether it appended
+// itself, so nobody reads the shared count while others append to it.  (Reading the
+// overflow flag from global memory and three barriers after every tile, with accumulator rows of 64-bit atomics:
+// 1M rows into 16 groups 33.0 -> 24.8 us, 100M Zipf rows into 3.8M groups 4.56 -> 3.26 ms.  The latter is bound by the
+// global table: about one random DRAM sector and three L2 operations per row that is not caught on chip.)
+// The first kHotKeys keys of a CTA also have kHotCopies copies of their accumulators, a lane's copy by its number:
+// with few groups most lanes of a warp meet in a few slots, and their shared atomics on one address run one
+// after another (eight queries of up to 2.5M rows into 100 groups: 172 -> 149 us).  A key's copies are used by the rows that see its number; the rows
+// before that went to its slot, and both are merged.
+// Shared memory: [S] key words | [n64][E] accumulators, E = S + kHotKeys * kHotCopies | multi-key [S][nk] key values | [B][rw]
+// buffer | multi-key [B][nk] key values | [n32][E] 32-bit counts | [S] key numbers (bytes, 255: none).
+constexpr int kHotKeys = 16, kHotCopies = 8;
 template <class Ev>
 __device__ void aggHash(const Launch& L) {
   extern __shared__ __align__(16) u64 wsSmem[];
-  __shared__ int spillN, stopFlag;
+  __shared__ int spillN, stopFlag, keysN;
   Ev ev(L);
   const int rw = ev.rowWords(), nk = ev.nk();
   const int S = L.smemSlots, B = L.spillRows;
   const bool multi = nk > 1;
-  u64* tab = wsSmem;
-  double* skv = (double*)(tab + (size_t)S * rw);
-  u64* buf = tab + (size_t)S * rw + (multi ? (size_t)S * nk : 0);
+  int n64, n32;
+  compactWords(ev, n64, n32);
+  u64* tkey = wsSmem;
+  u64* t64 = tkey + S;
+  const int E = S ? S + kHotKeys * kHotCopies : 0;
+  double* skv = (double*)(t64 + (size_t)E * n64);
+  u64* buf = (u64*)skv + (multi ? (size_t)S * nk : 0);
   double* bkv = (double*)(buf + (size_t)B * rw);
-  for (int s = threadIdx.x; s < S; s += blockDim.x) {
-    u64* row = tab + (size_t)s * rw;
-    rowIdentity(ev, row);
-    row[0] = kEmpty;
+  unsigned* t32 = (unsigned*)(bkv + (multi ? (size_t)B * nk : 0));
+  unsigned char* number = (unsigned char*)(t32 + (size_t)E * n32);
+  for (int e = threadIdx.x; e < E; e += blockDim.x) {
+    if (e < S) tkey[e] = kEmpty, number[e] = 255;
+    compactIdentity(ev, t64, t32, e, E);
   }
-  if (threadIdx.x == 0) spillN = 0;
+  if (threadIdx.x == 0) spillN = 0, keysN = 0;
   __syncthreads();
   const int lane = threadIdx.x & 31;
+  bool appended = false;  // this thread sent a row to the buffer since the last flush
   auto rowFn = [&](int i, int, i64) {
     double kv[Ev::NK];
     const u64 kw = keyWord(ev, i, kv);
     u64 x[kMaxRowWords];
     rowOfInput(ev, i, x);
-    if (kw != kEmpty && S > 0) {
+    if (kw != kEmpty && S > 0 && compactOk(L, ev, x, i)) {
       unsigned s = (unsigned)(mix64(kw) & (u64)(S - 1));
 #pragma unroll 1
       for (int p = 0; p < 8; ++p) {
-        u64* row = tab + (size_t)s * rw;
-        u64 prev = row[0];
+        u64 prev = *(volatile u64*)(tkey + s);
         if (prev == kEmpty) {
-          prev = atomicCAS(row, kEmpty, kw);
+          prev = atomicCAS(tkey + s, kEmpty, kw);
           if (prev == kEmpty) {
             if (multi)
               for (int k = 0; k < nk; ++k) skv[(size_t)s * nk + k] = kv[k];
+            const int num = *(volatile int*)&keysN < kHotKeys ? atomicAdd(&keysN, 1) : kHotKeys;
+            if (num < kHotKeys) *(volatile unsigned char*)(number + s) = (unsigned char)num;
             prev = kw;
           }
         }
         if (prev == kw) {
-          rowAtomicCombine(ev, row, x);
+          const unsigned num = *(volatile unsigned char*)(number + s);
+          const unsigned e = num < kHotKeys ? S + num * kHotCopies + (lane & (kHotCopies - 1)) : s;
+          compactAdd(ev, x, t64, t32, e, E);
           return;
         }
         s = (s + 1) & (S - 1);
@@ -830,94 +1112,71 @@ __device__ void aggHash(const Launch& L) {
     if (lane == leader) base = atomicAdd(&spillN, __popc(m));
     base = __shfl_sync(m, base, leader);
     const int at = base + rank;
+    appended = true;
     if (at < B) {
       u64* e = buf + (size_t)at * rw;
       for (int w = 1; w < rw; ++w) e[w] = x[w];
       e[0] = kw;
       if (multi)
         for (int k = 0; k < nk; ++k) bkv[(size_t)at * nk + k] = kv[k];
-    } else {
-      globalInsert(L, ev, kw, kv, x);
+    } else if (!*(volatile int*)(L.err + 1)) {
+      globalInsert(L, ev, kw, kv, x, globalPeek(L, ev, kw));
     }
   };
-  // Inserts the buffered rows; returns true (in every thread) once the global table has overflowed:
-  // the run's result is discarded then (the caller reruns with a bigger table), so the CTA stops.
-  // Barriers: the count and the flag are read between the first two, so no thread changes them (the
-  // next tile's appends, the next flush's flag) before every thread has read them: the decisions
-  // below are CTA-uniform.
-  auto flush = [&]() -> bool {
+  // Inserts the buffered rows (force: however few); returns true (in every thread) once the global table has
+  // overflowed: the run's result is discarded then (the caller reruns with a bigger table), so the CTA stops.
+  auto flush = [&](bool force) -> bool {
+    if (!__syncthreads_or(appended || force)) return false;
+    // every thread is past its appends and none appends before the last barrier below
+    const int n = min(spillN, B);
     if (threadIdx.x == 0) stopFlag = *(volatile int*)(L.err + 1);
     __syncthreads();
-    const int n = min(spillN, B);
-    const bool stop = stopFlag != 0;
-    __syncthreads();
-    if (n == 0 || stop) return stop;
     if (threadIdx.x == 0) spillN = 0;
-    for (int j = threadIdx.x; j < n; j += blockDim.x) {
-      const u64* e = buf + (size_t)j * rw;
-      double kv[WS_MAX_KEYS];
-      if (multi)
-        for (int k = 0; k < nk; ++k) kv[k] = bkv[(size_t)j * nk + k];
-      else
-        kv[0] = __longlong_as_double((i64)e[0]);
-      globalInsert(L, ev, e[0], kv, e);
-    }
+    appended = false;
+    if (stopFlag) return true;
+    insertAll(
+        L, ev, n, [&](int j) { return buf[(size_t)j * rw]; },
+        [&](int j, u64 kw, u64 first) {
+          const u64* e = buf + (size_t)j * rw;
+          double kv[WS_MAX_KEYS];
+          if (multi)
+            for (int k = 0; k < nk; ++k) kv[k] = bkv[(size_t)j * nk + k];
+          globalInsert(L, ev, kw, kv, e, first);
+        });
     __syncthreads();  // the buffer is refilled by the next tile
     return false;
   };
-  forEachRowTiles(L, ev, rowFn, flush);
-  if (flush()) return;  // overflowed: the shared table is not merged either
-  __syncthreads();
-  for (int s = threadIdx.x; s < S; s += blockDim.x) {
-    const u64* row = tab + (size_t)s * rw;
-    if (row[0] == kEmpty) continue;
-    double kv[WS_MAX_KEYS];
-    if (multi)
-      for (int k = 0; k < nk; ++k) kv[k] = skv[(size_t)s * nk + k];
-    else
-      kv[0] = __longlong_as_double((i64)row[0]);
-    globalInsert(L, ev, row[0], kv, row);
-  }
+  forEachRowTiles(L, ev, rowFn, [&]() { return flush(false); });
+  if (flush(true)) return;  // overflowed: the shared table is not merged either
+  insertAll(
+      L, ev, S, [&](int s) { return tkey[s]; },
+      [&](int s, u64 kw, u64 first) {
+        if (kw == kEmpty) return;
+        double kv[WS_MAX_KEYS];
+        if (multi)
+          for (int k = 0; k < nk; ++k) kv[k] = skv[(size_t)s * nk + k];
+        u64 w[kMaxRowWords];
+        rowIdentity(ev, w);
+        compactInto(ev, w, t64, t32, s, E);
+        if (number[s] < kHotKeys)
+          for (int c = 0; c < kHotCopies; ++c) compactInto(ev, w, t64, t32, S + number[s] * kHotCopies + c, E);
+        globalInsert(L, ev, kw, kv, w, first);
+      });
 }
 
 // ------------------------------------------------------------------ selection
-// Pass 1: selected rows per tile.  Pass 2 (after an exclusive scan of the tile counts): each warp
-// ranks its rows with ballot / popc and writes ascending global row indices.
+// One pass over the predicate's columns: a bit per row in selMask (32 words per tile, row r of the tile at bit r % 32 of
+// word r / 32) and the selected rows per tile.  The indices are written from the mask (kSelectWrite,
+// ws_select_join.cu) after a scan of the tile counts.
 template <class Ev>
-__device__ void selectCount(const Launch& L) {
-  __shared__ int wcount[kThreads / 32];
+__device__ void selectMask(const Launch& L) {
+  __shared__ int cnt[2];
   Ev ev(L);
+  const int lane = threadIdx.x & 31;
+  if (threadIdx.x < 2) cnt[threadIdx.x] = 0;
+  __syncthreads();
+  int turn = 0;
   forEachOwnedTile(L, ev, [&](i64 t, int, i64 r0, i64 n, const uint32_t* del) {
-    int c = 0;
-    if (r0 < n) {
-      const int nv = n - r0 >= 4 ? 4 : (int)(n - r0);
-      ev.load(r0, ev.fastOk && nv == 4, nv);
-      unsigned live = (1u << nv) - 1;
-      if (del) live &= ~(__ldg(del + (r0 >> 5)) >> (r0 & 31)) & 0xfu;
-#pragma unroll
-      for (int i = 0; i < 4; ++i) c += ((live >> i) & 1u) && ev.where(i);
-    }
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) c += __shfl_down_sync(0xffffffffu, c, o);
-    if ((threadIdx.x & 31) == 0) wcount[threadIdx.x >> 5] = c;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-      int s = 0;
-      for (int w = 0; w < kThreads / 32; ++w) s += wcount[w];
-      L.tileCount[t] = s;
-    }
-    __syncthreads();
-    return false;
-  });
-  ev.finish();
-}
-
-template <class Ev>
-__device__ void selectWrite(const Launch& L) {
-  __shared__ int woff[kThreads / 32];
-  Ev ev(L);
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  forEachOwnedTile(L, ev, [&](i64 t, int b, i64 r0, i64 n, const uint32_t* del) {
     unsigned sel = 0;
     if (r0 < n) {
       const int nv = n - r0 >= 4 ? 4 : (int)(n - r0);
@@ -928,26 +1187,16 @@ __device__ void selectWrite(const Launch& L) {
       for (int i = 0; i < 4; ++i)
         if (((live >> i) & 1u) && ev.where(i)) sel |= 1u << i;
     }
-    // rank = selected rows of lower lanes (ballot per row position) + own earlier rows
-    const unsigned lower = (1u << lane) - 1;
-    int before = 0, total = 0;
+    unsigned word = sel << (4 * (lane & 7));
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      const unsigned m = __ballot_sync(0xffffffffu, (sel >> i) & 1u);
-      before += __popc(m & lower);
-      total += __popc(m);
-    }
-    if (lane == 0) woff[warp] = total;
+    for (int o = 1; o < 8; o <<= 1) word |= __shfl_xor_sync(0xffffffffu, word, o);
+    if ((lane & 7) == 0) L.selMask[t * (kTile / 32) + threadIdx.x / 8] = word;
+    const int c = __reduce_add_sync(0xffffffffu, __popc(sel));
+    if (lane == 0 && c) atomicAdd(&cnt[turn], c);
     __syncthreads();
-    int base = 0;
-    for (int w = 0; w < warp; ++w) base += woff[w];
-    const i64 out0 = L.tileCount[t] + base + before;
-    const i64 g0 = __ldg(L.rowStart + b) + r0;
-    int k = 0;
-#pragma unroll
-    for (int i = 0; i < 4; ++i)
-      if ((sel >> i) & 1u) L.outIdx[out0 + k++] = (int32_t)(g0 + i);
-    __syncthreads();
+    // cnt[turn] is next added to two tiles on, after the next barrier, which thread 0 reaches behind this
+    if (threadIdx.x == 0) L.tileCount[t] = cnt[turn], cnt[turn] = 0;
+    turn ^= 1;
     return false;
   });
   ev.finish();
@@ -981,7 +1230,8 @@ __device__ void selectWrite(const Launch& L) {
     __syncthreads();                                                                                         \
     BODY(Lq);                                                                                                \
   }
-#define WS_K_MULTI_NOKEYS(EV, PREFIX) WS_K_MULTI_B(PREFIX, nokeys, ws::aggNoKeys<EV>, ws::kStagedThreads, 1)
+#define WS_K_MULTI_NOKEYS(EV, PREFIX) \
+  WS_K_MULTI_B(PREFIX, nokeys, (ws::aggNoKeys<EV, false>), ws::kThreads, EV::NOKEYS_MIN_BLOCKS)
 #define WS_K_MULTI_DENSE_PRIV(EV, PREFIX) \
   WS_K_MULTI_B(PREFIX, dense_priv, (ws::aggDensePriv<EV, false>), ws::kThreads, EV::PRIV_MIN_BLOCKS)
 // The hash scan launches kThreads.  For generated plans EV::HASH_MULTI_MIN_BLOCKS = 3 resident CTAs
@@ -990,22 +1240,17 @@ __device__ void selectWrite(const Launch& L) {
 // single-query scan; bounded it needs 80, without spills.
 #define WS_K_MULTI_HASH(EV, PREFIX) \
   WS_K_MULTI_B(PREFIX, hash, ws::aggHash<EV>, ws::kThreads, EV::HASH_MULTI_MIN_BLOCKS)
-#define WS_K_NOKEYS(EV, PREFIX) WS_K_ENTRY(PREFIX, nokeys, ws::aggNoKeys<EV>)
-#define WS_K_DENSE_SHARED(EV, PREFIX) WS_K_ENTRY(PREFIX, dense_shared, ws::aggDenseShared<EV>)
+// Direct loads: EV::NOKEYS_MIN_BLOCKS resident CTAs of kThreads; the staged entry keeps the producer warp.
+#define WS_K_NOKEYS(EV, PREFIX) \
+  WS_K_ENTRY_B(PREFIX, nokeys, (ws::aggNoKeys<EV, false>), ws::kThreads, EV::NOKEYS_MIN_BLOCKS)
+#define WS_K_NOKEYS_STAGED(EV, PREFIX) WS_K_ENTRY(PREFIX, nokeys_staged, (ws::aggNoKeys<EV, true>))
+#define WS_K_DENSE_SHARED(EV, PREFIX) \
+  WS_K_ENTRY_B(PREFIX, dense_shared, ws::aggDenseShared<EV>, (ws::kThreads * EV::DENSE_V), 1)
 #define WS_K_DENSE_GLOBAL(EV, PREFIX) WS_K_ENTRY(PREFIX, dense_global, ws::aggDenseGlobal<EV>)
 // The direct-load private-row kernel asks for EV::PRIV_MIN_BLOCKS resident CTAs of kThreads (a
 // register budget); the staged one keeps the producer warp.
 #define WS_K_DENSE_PRIV(EV, PREFIX)                                                                      \
-  WS_K_ENTRY_B(PREFIX, dense_priv, (ws::aggDensePriv<EV, false>), ws::kThreads, EV::PRIV_MIN_BLOCKS)     \
-  WS_K_ENTRY(PREFIX, dense_priv_staged, (ws::aggDensePriv<EV, true>))
-#define WS_K_HASH(EV, PREFIX) WS_K_ENTRY(PREFIX, hash, ws::aggHash<EV>)
-#define WS_K_SELECT_COUNT(EV, PREFIX) WS_K_ENTRY(PREFIX, select_count, ws::selectCount<EV>)
-#define WS_K_SELECT_WRITE(EV, PREFIX) WS_K_ENTRY(PREFIX, select_write, ws::selectWrite<EV>)
-#define WS_DEFINE_SCAN_KERNELS(EV, PREFIX) \
-  WS_K_NOKEYS(EV, PREFIX)                  \
-  WS_K_DENSE_SHARED(EV, PREFIX)            \
-  WS_K_DENSE_GLOBAL(EV, PREFIX)            \
-  WS_K_DENSE_PRIV(EV, PREFIX)              \
-  WS_K_HASH(EV, PREFIX)                    \
-  WS_K_SELECT_COUNT(EV, PREFIX)            \
-  WS_K_SELECT_WRITE(EV, PREFIX)
+  WS_K_ENTRY_B(PREFIX, dense_priv, (ws::aggDensePriv<EV, false>), ws::kThreads, EV::PRIV_MIN_BLOCKS)
+#define WS_K_DENSE_PRIV_STAGED(EV, PREFIX) WS_K_ENTRY(PREFIX, dense_priv_staged, (ws::aggDensePriv<EV, true>))
+#define WS_K_HASH(EV, PREFIX) WS_K_ENTRY_B(PREFIX, hash, ws::aggHash<EV>, ws::kThreads, EV::HASH_MIN_BLOCKS)
+#define WS_K_SELECT(EV, PREFIX) WS_K_ENTRY_B(PREFIX, select, ws::selectMask<EV>, ws::kThreads, EV::SELECT_MIN_BLOCKS)

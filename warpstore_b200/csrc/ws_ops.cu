@@ -23,6 +23,7 @@ const KernelSet& interpKernels() {
     interpSyms_select(syms);
     for (int i = 0; i < K_COUNT_; ++i) {
       cudaFunction_t f;
+      if (!syms[i]) continue;  // staged kernels: compiled plans only
       WS_CK(cudaGetFuncBySymbol(&f, syms[i]));
       k.fn[i] = (CUfunction)f;
     }
@@ -133,7 +134,7 @@ __device__ __forceinline__ double keyOut(const ResultSpec& s, int64_t i, int k) 
     const long long v = s.kmin[k] + (i / s.stride[k]) % s.range[k];
     return s.keyInt[k] ? __longlong_as_double(v) : (double)v;
   }
-  if (s.nk == 1 && i != s.cap) return __longlong_as_double((long long)s.rows[i * s.rw]);
+  if (s.nk == 1) return __longlong_as_double(i == s.cap ? (long long)kEmpty : (long long)s.rows[i * s.rw]);
   return s.tkeys[i * s.nk + k];
 }
 // Exact words of slot a of result row i: (lo, hi) of an integer SUM, (value, 0) otherwise.
@@ -548,34 +549,56 @@ static void aggResetRows(ws_aggregator& A) {
 
 static void aggInitRows(ws_aggregator& A) {
   const int64_t nr = A.nrows();
-  A.rows = DBuf<u64>(nr * A.lay.rw + kCtlWords);
-  if (A.plan.nkeys && !A.isDense) {
-    A.tkeys = DBuf<double>((A.cap + 1) * std::max(A.plan.nkeys, 1));
-  }
+  const int64_t words = nr * A.lay.rw + kCtlWords;
+  A.rows = DBuf<u64>((u64*)tableAlloc(8 * (size_t)words), words);
+  // key values beside the table: several keys only (a single key is its key word, in the extra row too: the empty
+  // marker's bits)
+  if (A.plan.nkeys > 1 && !A.isDense) A.tkeys = DBuf<double>((A.cap + 1) * A.plan.nkeys);
   aggResetRows(A);
 }
 
 static TuneChoice tuneScan(ws_aggregator& A, const std::string& key, const std::vector<TuneChoice>& cands,
                            const std::function<void(const TuneChoice&)>& launch);
 
-// Default shared-memory budget of the hash scan's per-CTA table (KB; WARPSTORE_B200_HASH_SMEM_KB).
-// 48 KB (1024 slots of a 32-byte row, 3 CTAs per SM with the spill buffer) measured 28 % faster than
-// 64 KB on 100M Zipf-keyed rows (4.89 vs 6.79 ms) and the same on 16 groups, 6 groups and the
-// serving workload's multi-key queries.
-static int hashTableKB() {
+// Shared-memory budget of the hash scan's per-CTA table in bytes (WARPSTORE_B200_HASH_SMEM_KB overrides).  Where a
+// table of half the global table's capacity (capacities are chosen at twice the expected groups) fits 52 KB the CTA
+// keeps about every group on chip; a table of the whole capacity only costs (eight queries into 100 groups: 178
+// against 149 us).  Beyond that the table catches hot keys and the scan waits for the global table, so resident
+// warps count more than slots: with 24 KB, and as much for the spill buffer, four CTAs fit an SM (100M Zipf rows:
+// 48 + 40 KB and two CTAs 5.39 ms, 24 + 32 KB 3.57 ms, 24 + 24 KB 3.23 ms; 24 + 8 KB overflows into single inserts:
+// 4.90 ms).
+static size_t hashTableBytes(const ws_aggregator& A, size_t slots, bool compact);
+constexpr size_t kHashFitBytes = 52 * 1024, kHashHotBytes = 24 * 1024, kHashSpillBytes = 24 * 1024;
+static size_t hashTableBudget(const ws_aggregator& A, bool compact) {
   static const int kb = [] {
     const char* e = getenv("WARPSTORE_B200_HASH_SMEM_KB");
     const int v = e ? atoi(e) : 0;
-    return v >= 4 && v <= 160 ? v : 48;
+    return v >= 4 && v <= 160 ? v : 0;
   }();
-  return kb;
+  if (kb) return (size_t)kb * 1024;
+  const int64_t s = std::max<int64_t>(A.cap / 2, 64);
+  if (s <= 4096 && hashTableBytes(A, (size_t)s, compact) <= kHashFitBytes) return hashTableBytes(A, (size_t)s, compact);
+  return kHashHotBytes;
 }
 
-static size_t hashSmemSlots(const ws_aggregator& A, size_t budget) {
-  const size_t per = (size_t)A.lay.rw * 8 + (A.plan.nkeys > 1 ? (size_t)A.plan.nkeys * 8 : 0);
+// Bytes of a group's compact accumulators (ws_kern.cuh), and of the hash scan's shared table of `slots` slots: key word,
+// accumulators (also the hot keys' copies), key number, key values of several keys.
+// compact: compiled plans; the interpreter keeps accumulator rows.
+static size_t compactBytes(const ws_aggregator& A, bool compact) {
+  size_t b = 0;
+  if (!compact) return (size_t)A.lay.rw * 8;
+  for (int a = 0; a < A.lay.na; ++a) b += A.lay.kind[a] == SK_COUNT ? 4 : A.lay.kind[a] != SK_NONE ? 8 : 0;
+  return b;
+}
+static size_t hashTableBytes(const ws_aggregator& A, size_t slots, bool compact) {
+  if (!slots) return 0;
+  return slots * (9 + compactBytes(A, compact) + (A.plan.nkeys > 1 ? (size_t)A.plan.nkeys * 8 : 0)) +
+         kHotKeys * kHotCopies * compactBytes(A, compact);
+}
+static size_t hashSmemSlots(const ws_aggregator& A, size_t budget, bool compact) {
   size_t s = 4096;
-  while (s > 64 && s * per > budget) s >>= 1;
-  return s * per > budget ? 0 : s;
+  while (s > 64 && hashTableBytes(A, s, compact) > budget) s >>= 1;
+  return hashTableBytes(A, s, compact) > budget ? 0 : s;
 }
 
 // A scan prepared for launching elsewhere (a captured graph): kernel, shape, launch descriptor and the
@@ -584,6 +607,8 @@ struct PreparedScan {
   bool direct = false;    // in: direct loads only (a multi-query launch has no staged form)
   bool ready = false;     // false: the batches hold no tiles (nothing to launch)
   bool compiled = false;  // the plan's generated kernels (not the interpreter)
+  bool hot = false;       // of the evaluator of hinted storage (ws_jit_program::kernels)
+  int scan = -1;          // the scan kind's KernelId
   CUfunction f = nullptr;
   unsigned grid = 0;
   size_t smem = 0;
@@ -614,7 +639,8 @@ static void aggRun(ws_aggregator& A, const ws_expr_env& env, const ws_jit_progra
   L.rows = A.rows.p;
   L.err = A.err();
   L.ticket = A.ticket();
-  const KernelSet& ks = useJit ? jit->kernels : interpKernels();
+  const KernelSet& ks = useJit ? jit->kernelsFor(nb, A.ncols, A.bcols.data()) : interpKernels();
+  const KernelSet& anyStorage = useJit ? jit->generic : ks;  // staged kernels
   // Staged scans: a ring of 2..4 tile stages in shared memory (compiled plans only).
   const int stageBytes = useJit ? jit->stageBytes : 0;
   static const int maxStages = [] {  // WARPSTORE_B200_STAGES: shared-memory tile stages (0: direct loads,
@@ -634,6 +660,7 @@ static void aggRun(ws_aggregator& A, const ws_expr_env& env, const ws_jit_progra
   std::function<Shape(const TuneChoice&)> shapeOf;
   const char* name = "";
   int64_t partRows = 0;  // rows of `part` per CTA (0: none)
+  int tilesPerCta = 1;   // tiles a CTA visits at a time
   std::vector<TuneChoice> cands(1);  // candidates for the autotuner; [0] = the default shape
   auto ctas = [](int c) {
     TuneChoice t;
@@ -647,15 +674,15 @@ static void aggRun(ws_aggregator& A, const ws_expr_env& env, const ws_jit_progra
   };
   Launch* lp = &L;
   if (A.plan.nkeys == 0) {
-    CUfunction f = ks.fn[K_NOKEYS];
+    CUfunction f = ks.fn[K_NOKEYS], stagedFn = anyStorage.fn[K_NOKEYS_STAGED];
     if (!f) throw Error("compiled plan has no aggregation kernel", WS_ERR_INTERNAL);
     shapeOf = [=](const TuneChoice& c) {
       // stage count: the choice's, else the default; within 200 KB of tile stages
       int st = c.stages >= 0 ? c.stages : S;
       if (stageBytes > 0) st = (int)std::min<int64_t>(st, (200 * 1024) / stageBytes);
-      if (st < 2 || stageBytes <= 0) st = 0;
+      if (st < 2 || stageBytes <= 0 || !stagedFn) st = 0;
       lp->stages = st;
-      return Shape{f, (size_t)st * stageBytes, st ? kStagedThreads : kThreads};
+      return Shape{st ? stagedFn : f, (size_t)st * stageBytes, st ? kStagedThreads : kThreads};
     };
     name = "nokeys";
     partRows = 1;
@@ -671,17 +698,29 @@ static void aggRun(ws_aggregator& A, const ws_expr_env& env, const ws_jit_progra
       L.stride[k] = A.dense.stride[k];
     }
     L.G = A.dense.G;
+    L.kmin32 = 1;
+    for (int k = 0; k < A.plan.nkeys; ++k)
+      if (A.dense.kmin[k] > (1 << 30) || A.dense.kmin[k] < -(1 << 30)) L.kmin32 = 0;
     const int64_t G = A.dense.G;
     // few groups: private register rows per thread in shared memory (+ staged tiles when they fit)
     // private rows [G][frw][kThreads] + int128 spill counters [G][NA][2] (NA: the evaluator's slot bound)
     const int naEv = ks.interp ? WS_INTERP_AGGS : A.plan.naggs;
     const size_t privBytes = (size_t)G * A.lay.frw * kThreads * 8 + (size_t)G * naEv * 16;
-    const size_t sharedSmem = (size_t)G * A.lay.rw * 8;
+    // compact accumulators per group (ws_kern.cuh), in copies while they are small: few groups meet in a warp
+    const size_t groupBytes = compactBytes(A, !ks.interp);
+    int copies = 1;
+    while (!ks.interp && copies < 8 && (size_t)G * copies * 2 * groupBytes <= 24 * 1024) copies <<= 1;
+    const size_t sharedSmem = (size_t)G * copies * groupBytes;
+    // A table an SM holds once pays when the CTA brings the SM's warps with it (denseV: 5000 groups of 24 B, 12M rows:
+    // 83 us against 377 us of L2 atomics), and where the rows well outnumber the groups each CTA merges
+    const int denseV = ks.denseV;
+    const size_t sharedLimit = denseV > 1 ? 200 * 1024 : 96 * 1024;
+    const bool sharedPays = sharedSmem <= 48 * 1024 || d.rows >= 16 * G;
     if (G * A.lay.frw <= 48 && ks.fn[K_DENSE_PRIV]) {
       // tile stages fit beside the private rows within 220 KB; the staged body is its own entry
       const int64_t room = std::max<int64_t>(0, (int64_t)(220 * 1024) - (int64_t)privBytes);
       const int fitStages = stageBytes > 0 ? (int)std::min<int64_t>(8, room / stageBytes) : 0;
-      CUfunction direct = ks.fn[K_DENSE_PRIV], stagedFn = ks.fn[K_DENSE_PRIV_STAGED];
+      CUfunction direct = ks.fn[K_DENSE_PRIV], stagedFn = anyStorage.fn[K_DENSE_PRIV_STAGED];
       shapeOf = [=](const TuneChoice& c) {
         int st = std::min(c.stages >= 0 ? c.stages : maxStages, fitStages);
         if (st < 2 || !stagedFn) st = 0;
@@ -695,9 +734,11 @@ static void aggRun(ws_aggregator& A, const ws_expr_env& env, const ws_jit_progra
         for (int st : {0, 2, 3})
           if (st <= fitStages && st != (std::min(maxStages, fitStages) >= 2 ? std::min(maxStages, fitStages) : 0))
             cands.push_back(staged(st));
-    } else if (sharedSmem <= 96 * 1024 && ks.fn[K_DENSE_SHARED]) {
+    } else if (sharedSmem <= sharedLimit && sharedPays && ks.fn[K_DENSE_SHARED]) {
       CUfunction f = ks.fn[K_DENSE_SHARED];
-      shapeOf = [=](const TuneChoice&) { return Shape{f, sharedSmem, kThreads}; };
+      L.copies = copies;
+      tilesPerCta = denseV;
+      shapeOf = [=](const TuneChoice&) { return Shape{f, sharedSmem, kThreads * denseV}; };
       name = "dense_shared";
       cands.push_back(ctas(2));
       cands.push_back(ctas(1));
@@ -718,14 +759,14 @@ static void aggRun(ws_aggregator& A, const ws_expr_env& env, const ws_jit_progra
     L.count = A.count();
     L.probeLimit = (int)std::min<int64_t>(A.cap, 1 << 16);
     const size_t per = (size_t)A.lay.rw * 8 + (A.plan.nkeys > 1 ? (size_t)A.plan.nkeys * 8 : 0);
-    // spill buffer: up to a tile's rows, within 40 KB
-    L.spillRows = (int)std::min<size_t>(kTile, (40 * 1024) / per);
+    L.spillRows = (int)std::min<size_t>(kTile, kHashSpillBytes / per);
     ws_aggregator* ap = &A;
+    const bool compact = !ks.interp;
     shapeOf = [=](const TuneChoice& c) {
-      // per-CTA table: up to 4096 slots within the budget (default 64 KB)
-      const size_t slots = hashSmemSlots(*ap, (size_t)(c.smemKB > 0 ? c.smemKB : hashTableKB()) * 1024);
+      // per-CTA table: up to 4096 slots within the budget
+      const size_t slots = hashSmemSlots(*ap, c.smemKB > 0 ? (size_t)c.smemKB * 1024 : hashTableBudget(*ap, compact), compact);
       lp->smemSlots = (int)slots;
-      return Shape{f, (slots + (size_t)lp->spillRows) * per, kThreads};
+      return Shape{f, hashTableBytes(*ap, slots, compact) + (size_t)lp->spillRows * per, kThreads};
     };
     name = "hash";
     for (int kb : {16, 32, 96}) {
@@ -739,7 +780,7 @@ static void aggRun(ws_aggregator& A, const ws_expr_env& env, const ws_jit_progra
   int64_t partCap = 0;
   auto launchOnce = [&](const TuneChoice& c) {
     const Shape sh = shapeOf(c);
-    unsigned grid = persistentGrid(sh.f, sh.smem, d.ntiles, sh.threads);
+    unsigned grid = persistentGrid(sh.f, sh.smem, (d.ntiles + tilesPerCta - 1) / tilesPerCta, sh.threads);
     if (c.ctasPerSm > 0) grid = (unsigned)std::max<int64_t>(1, std::min<int64_t>(grid, (int64_t)c.ctasPerSm * smCount()));
     if (partRows) {
       if ((int64_t)grid * partRows > partCap) {
@@ -765,7 +806,7 @@ static void aggRun(ws_aggregator& A, const ws_expr_env& env, const ws_jit_progra
   if (prep && prep->direct) choice.stages = 0;
   if (prep) {
     const Shape sh = shapeOf(choice);
-    unsigned grid = persistentGrid(sh.f, sh.smem, d.ntiles, sh.threads);
+    unsigned grid = persistentGrid(sh.f, sh.smem, (d.ntiles + tilesPerCta - 1) / tilesPerCta, sh.threads);
     if (choice.ctasPerSm > 0)
       grid = (unsigned)std::max<int64_t>(1, std::min<int64_t>(grid, (int64_t)choice.ctasPerSm * smCount()));
     if (partRows) {
@@ -773,6 +814,9 @@ static void aggRun(ws_aggregator& A, const ws_expr_env& env, const ws_jit_progra
       L.part = part.p;
     }
     prep->compiled = useJit;
+    prep->hot = useJit && &ks == &jit->kernels;
+    for (int k : {K_NOKEYS, K_DENSE_PRIV, K_HASH})
+      if (sh.f == ks.fn[k]) prep->scan = k;
     prep->f = sh.f;
     prep->grid = grid;
     prep->smem = sh.smem;
@@ -949,6 +993,9 @@ struct MultiPlan {
 
 static MultiPlan planMulti(const std::vector<const PreparedScan*>& preps, const ws_jit_program* jit, const char* who) {
   MultiPlan mp;
+  // queries whose batches all are stored as hinted run that evaluator's kernel, else all run the generic one
+  bool hot = true;
+  for (const PreparedScan* p : preps) hot = hot && (!p->ready || p->hot);
   const KernelSet* ks = nullptr;
   int multi = -1;
   int64_t tiles = 0;
@@ -956,9 +1003,10 @@ static MultiPlan planMulti(const std::vector<const PreparedScan*>& preps, const 
     const PreparedScan& p = *preps[i];
     if (!p.ready) continue;  // no tiles: nothing to scan
     if (p.compiled && !jit) throw Error(std::string(who) + ": compiled queries need their plan", WS_ERR_ARG);
-    const KernelSet& k = p.compiled ? jit->kernels : interpKernels();
-    const int m = p.f == k.fn[K_NOKEYS] ? K_MULTI_NOKEYS : p.f == k.fn[K_DENSE_PRIV] ? K_MULTI_DENSE_PRIV
-                : p.f == k.fn[K_HASH] ? K_MULTI_HASH : -1;
+    const KernelSet& own = !p.compiled ? interpKernels() : p.hot ? jit->kernels : jit->generic;
+    const KernelSet& k = !p.compiled ? interpKernels() : hot ? jit->kernels : jit->generic;
+    const int m = p.scan < 0 || p.f != own.fn[p.scan] ? -1
+                : p.scan == K_NOKEYS ? K_MULTI_NOKEYS : p.scan == K_DENSE_PRIV ? K_MULTI_DENSE_PRIV : K_MULTI_HASH;
     if (m < 0 || !k.fn[m] || p.L.stages)
       throw Error(std::string(who) + ": a query's scan has no multi-query form (dense shared / global rows, staged tiles)",
                   WS_ERR_ARG);

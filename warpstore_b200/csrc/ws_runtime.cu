@@ -98,6 +98,39 @@ void setStream(cudaStream_t s) {
   tStreamSet = s != nullptr;
 }
 
+// Large result tables have a stream-ordered pool of their own, per device.  In the default pool a 537 MB table freed by one
+// query was cut up by the next ones' smaller temporaries, and the driver mapped new memory for the next table: 0.3
+// to 110 ms per allocation in a loop of one high-cardinality query; from their own pool such tables come back whole
+// in microseconds.  What the pool keeps is bounded (an eighth of the device's memory) and given back like the default
+// pool's (ws_gpu_trim_pool, or when an allocation fails).
+namespace {
+constexpr int kMaxDevices = 64;
+std::mutex gTablePoolMu;
+cudaMemPool_t gTablePool[kMaxDevices] = {};
+cudaMemPool_t tablePool(bool create) {
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev >= kMaxDevices) return nullptr;
+  std::lock_guard<std::mutex> g(gTablePoolMu);
+  if (!gTablePool[dev] && create) {
+    cudaMemPoolProps props{};
+    props.allocType = cudaMemAllocationTypePinned;
+    props.location.type = cudaMemLocationTypeDevice;
+    props.location.id = dev;
+    cudaMemPool_t p = nullptr;
+    size_t fr = 0, total = 0;
+    if (cudaMemPoolCreate(&p, &props) != cudaSuccess || cudaMemGetInfo(&fr, &total) != cudaSuccess) {
+      cudaGetLastError();
+      if (p) cudaMemPoolDestroy(p);
+      return nullptr;
+    }
+    uint64_t keep = total / 8;
+    cudaMemPoolSetAttribute(p, cudaMemPoolAttrReleaseThreshold, &keep);
+    gTablePool[dev] = p;
+  }
+  return gTablePool[dev];
+}
+}  // namespace
+
 static void trimPool() {
   int dev = 0;
   cudaGetDevice(&dev);
@@ -105,7 +138,22 @@ static void trimPool() {
   if (cudaDeviceGetDefaultMemPool(&pool, dev) != cudaSuccess) return;
   cudaDeviceSynchronize();
   cudaMemPoolTrimTo(pool, 0);
+  if (cudaMemPool_t t = tablePool(false)) cudaMemPoolTrimTo(t, 0);
   cudaGetLastError();
+}
+
+void* tableAlloc(size_t bytes) {
+  constexpr size_t kLarge = 32u << 20;
+  ensureInit();
+  cudaMemPool_t pool = bytes >= kLarge ? tablePool(true) : nullptr;
+  if (!pool) return tmpAlloc(bytes);
+  void* p = nullptr;
+  if (cudaMallocFromPoolAsync(&p, bytes, pool, stream()) != cudaSuccess) {
+    cudaGetLastError();
+    trimPool();
+    WS_CK(cudaMallocFromPoolAsync(&p, bytes, pool, stream()));
+  }
+  return p;
 }
 
 void* tmpAlloc(size_t bytes) {
@@ -139,8 +187,9 @@ void countLaunch(int n) { gLaunches += n; }
 // instead: chunk i is copied by DMA into a ring slot while chunks already landed are copied out of
 // their slots by a small pool of host threads.
 namespace {
-constexpr size_t kRingChunk = 8u << 20;
-constexpr int kRingSlots = 4;
+// Chunks of 2 MB: results of a few MB pipeline too (an 8 MB copy into pageable memory took 0.4 ms by itself).
+constexpr size_t kRingChunk = 2u << 20;
+constexpr int kRingSlots = 8;
 struct PinnedRing {
   uint8_t* buf = nullptr;
   cudaEvent_t ev[kRingSlots] = {};
@@ -207,7 +256,7 @@ CopyPool& copyPool() {  // process-wide; never destroyed (its threads idle until
 }  // namespace
 
 void d2hLarge(void* h, const void* d, size_t b) {
-  if (b < 2 * kRingChunk) {
+  if (b < kRingChunk) {
     d2hSync(h, d, b);
     return;
   }
