@@ -506,7 +506,7 @@ static int hotDenseV(int words) { return words <= 28 ? 4 : 2; }
 //    row that raises a flag is evaluated again with the checked 64-bit operations.  The same results: a row
 //    without flags has the narrow value exactly, and its 64-bit operations could not have overflowed.
 // Pricing summary (60M rows): 0.587 -> 0.456 ms; selective scan over five encoded columns (30M rows): 0.730 -> 0.219 ms.
-// Empty when the plan has no such form (hints 7 / 8); *encs receives the (column, encoding) pairs it relies on.
+// Empty when the plan has no such form (hints 7 / 8, a vector column read as a value); *encs receives the (column, encoding) pairs it relies on.
 std::string genHot(const ws_expr_env& env, int ncols, const ws_agg_plan& plan, int fnKind,
                    std::vector<std::pair<int, int>>* encs, int* denseV) {
   Gen g{env, ncols};
@@ -543,7 +543,7 @@ std::string genHot(const ws_expr_env& env, int ncols, const ws_agg_plan& plan, i
   for (auto& [c, u] : g.cols) {
     const int e = env.cols[c].enc;
     if (u.vec) continue;
-    if (e >= 7) return "";
+    if (e >= 7 || u.t == 5) return "";
     const bool f64 = u.t == 2;
     if (e && f64 != (e >= 4)) return "";
     width[c] = e == 0 ? (u.t == 0 || u.t == 3 ? 4 : 8) : e == 1 || e == 4 ? 1 : e == 2 || e == 5 ? 2 : 4;
