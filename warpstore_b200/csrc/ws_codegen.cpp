@@ -29,6 +29,11 @@ std::atomic<int> gDefaultMode{WS_JIT_ON};
 thread_local int tMode = -1;
 std::mutex gMu;
 std::map<std::string, std::shared_ptr<ws_jit_program>> gCache;
+// The same programs by what their source is generated from (planShape), so that a query whose shape was seen before
+// is found without generating its evaluators again.  At most kMaxShapes entries (then emptied: a miss only
+// costs the generation).
+constexpr size_t kMaxShapes = 4096;
+std::map<std::string, std::shared_ptr<ws_jit_program>> gByShape;
 std::vector<std::shared_ptr<ws_jit_program>> gById;
 std::string gDiskDir;
 thread_local std::string tSql;
@@ -760,6 +765,23 @@ PlanSource planSource(const ws_expr_env& env, int ncols, const ws_agg_plan& plan
   return p;
 }
 
+// Everything the source of a plan is generated from, by value: the kind, the plan, the bytecode, and the columns'
+// types, scales and encoding hints (no constants, pointers or set / map contents).
+std::string planShape(const ws_expr_env& env, int ncols, const ws_agg_plan& plan, int fnKind) {
+  ws_agg_plan p;
+  memcpy(&p, &plan, sizeof p);
+  p.genv = nullptr;
+  std::string s;
+  s.reserve(sizeof p + sizeof env.code + 3 * WS_MAX_COLS + 8);
+  s.append((const char*)&fnKind, sizeof fnKind).append((const char*)&ncols, sizeof ncols);
+  s.append((const char*)&p, sizeof p).append((const char*)env.code, sizeof env.code);
+  for (int c = 0; c < WS_MAX_COLS; ++c) {
+    const char v[3] = {(char)env.cols[c].t, (char)env.cols[c].scale, (char)env.cols[c].enc};
+    s.append(v, 3);
+  }
+  return s;
+}
+
 uint64_t fnv64(const std::string& s, uint64_t h) {
   for (unsigned char c : s) h = (h ^ c) * 0x100000001b3ull;
   return h;
@@ -972,12 +994,18 @@ int ws_jit_get(const ws_expr_env* env, int ncols, const ws_agg_plan* plan, int f
     *out = nullptr;
     const int mode = jitMode();
     if (mode == WS_JIT_OFF) return;
-    const PlanSource src = planSource(*env, ncols, *plan, fn);
-    const std::string& ev = src.evaluators;
-    const std::string key = std::to_string(fn) + "\n" + ev;
+    const std::string shape = planShape(*env, ncols, *plan, fn);
     std::shared_ptr<ws_jit_program> p;
     bool fresh = false;
     {
+      std::lock_guard<std::mutex> g(gMu);
+      auto it = gByShape.find(shape);
+      if (it != gByShape.end()) p = it->second;
+    }
+    if (!p) {
+      const PlanSource src = planSource(*env, ncols, *plan, fn);
+      const std::string& ev = src.evaluators;
+      const std::string key = std::to_string(fn) + "\n" + ev;
       std::lock_guard<std::mutex> g(gMu);
       auto it = gCache.find(key);
       if (it != gCache.end()) {
@@ -998,6 +1026,8 @@ int ws_jit_get(const ws_expr_env* env, int ncols, const ws_agg_plan* plan, int f
         gCache.emplace(key, p);
         fresh = true;
       }
+      if (gByShape.size() >= kMaxShapes) gByShape.clear();
+      gByShape[shape] = p;
     }
     if (fresh) {
       if (mode == WS_JIT_SYNC) {
@@ -1121,6 +1151,7 @@ int ws_jit_clear_cache(void) {
   std::lock_guard<std::mutex> g(gMu);
   gById.clear();
   gCache.clear();
+  gByShape.clear();
   return WS_OK;
 }
 int ws_jit_begin_query(const char* sql) {
