@@ -524,7 +524,11 @@ WS_DI void slotCombine(int k, u64& lo, u64& hi, u64 l, u64 h) {
 // Reduces every (row, slot) of nrows rows over N contributors, one pair per warp at a time: lane l folds
 // contributors l, l + 32, ... in order, then a fixed shuffle tree combines the lanes (deterministic), and lane 0
 // calls put(row, slot, lo, hi).  get(row, slot, contributor, lo, hi) reads a value.  A pair moves its one or two
-// words only and needs no barrier, where whole rows went through every shuffle group by group.
+// words only and needs no barrier, where whole rows went through every shuffle group by group.  A lane reads
+// kPairLoads values before it combines them: a combination branches on the slot's kind, so a load behind it would
+// wait for the one before (1M rows, COUNT and two SUMs into 4 groups: 31.9 us that way, 23.5 us so; without GROUP BY
+// 14.0 and 10.7 us).
+constexpr int kPairLoads = 8;
 template <class Ev, class Get, class Put>
 WS_DI void reducePairs(const Ev& ev, int nrows, int N, Get&& get, Put&& put) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5, na = ev.na();
@@ -533,11 +537,14 @@ WS_DI void reducePairs(const Ev& ev, int nrows, int N, Get&& get, Put&& put) {
     if (k == SK_NONE) continue;
     u64 lo, hi;
     slotIdentity(k, lo, hi);
-#pragma unroll 4
-    for (int c = lane; c < N; c += 32) {
-      u64 l, h;
-      get(r, a, c, l, h);
-      slotCombine(k, lo, hi, l, h);
+    for (int c0 = lane; c0 < N; c0 += 32 * kPairLoads) {
+      u64 l[kPairLoads], h[kPairLoads];
+#pragma unroll
+      for (int j = 0; j < kPairLoads; ++j)
+        if (c0 + 32 * j < N) get(r, a, c0 + 32 * j, l[j], h[j]);
+#pragma unroll
+      for (int j = 0; j < kPairLoads; ++j)
+        if (c0 + 32 * j < N) slotCombine(k, lo, hi, l[j], h[j]);
     }
 #pragma unroll
     for (int off = 16; off > 0; off >>= 1) {
