@@ -55,6 +55,7 @@ cudaStream_t stream();           // the calling thread's stream (ws_set_stream),
 void* tmpAlloc(size_t bytes);    // stream-ordered pool allocation on stream()
 void* tableAlloc(size_t bytes);  // the same for result tables: large ones from a pool of their own (freed by tmpFree)
 void tmpFree(void* p);
+void trimPool();                 // returns what the pools hold unused to the device (synchronises)
 void h2dAsync(void* d, const void* h, size_t b);
 void d2hSync(void* h, const void* d, size_t b);
 // The same for large copies into pageable memory: pipelined through pinned staging (synchronous).

@@ -101,8 +101,9 @@ void setStream(cudaStream_t s) {
 // Large result tables have a stream-ordered pool of their own, per device.  In the default pool a 537 MB table freed by one
 // query was cut up by the next ones' smaller temporaries, and the driver mapped new memory for the next table: 0.3
 // to 110 ms per allocation in a loop of one high-cardinality query; from their own pool such tables come back whole
-// in microseconds.  What the pool keeps is bounded (an eighth of the device's memory) and given back like the default
-// pool's (ws_gpu_trim_pool, or when an allocation fails).
+// in microseconds.  The pool serves tables while they fit an eighth of the device's memory together, so what it keeps is
+// bounded and never unmapped at a synchronisation; further tables come from the default pool.  Both are given back
+// alike: by ws_gpu_trim_pool, and when an allocation or a column's placement finds no memory.
 namespace {
 constexpr int kMaxDevices = 64;
 std::mutex gTablePoolMu;
@@ -131,7 +132,7 @@ cudaMemPool_t tablePool(bool create) {
 }
 }  // namespace
 
-static void trimPool() {
+void trimPool() {
   int dev = 0;
   cudaGetDevice(&dev);
   cudaMemPool_t pool;
@@ -146,7 +147,13 @@ void* tableAlloc(size_t bytes) {
   constexpr size_t kLarge = 32u << 20;
   ensureInit();
   cudaMemPool_t pool = bytes >= kLarge ? tablePool(true) : nullptr;
-  if (!pool) return tmpAlloc(bytes);
+  uint64_t used = 0, keep = 0;
+  if (pool && (cudaMemPoolGetAttribute(pool, cudaMemPoolAttrUsedMemCurrent, &used) != cudaSuccess ||
+               cudaMemPoolGetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep) != cudaSuccess)) {
+    cudaGetLastError();
+    pool = nullptr;
+  }
+  if (!pool || used + bytes > keep) return tmpAlloc(bytes);
   void* p = nullptr;
   if (cudaMallocFromPoolAsync(&p, bytes, pool, stream()) != cudaSuccess) {
     cudaGetLastError();

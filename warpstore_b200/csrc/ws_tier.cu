@@ -169,15 +169,8 @@ int ws_place_column(void* host, size_t bytes, int host_only, void** out, int* ma
     if (!bytes) return;
     if (!host_only && fits(bytes)) {
       void* p = countedAlloc(bytes);
-      if (!p) {  // memory the pool holds may be returned to the device
-        WS_CK(cudaDeviceSynchronize());
-        WS_CK(cudaMemPoolTrimTo([] {
-          cudaMemPool_t pool;
-          int dev = 0;
-          cudaGetDevice(&dev);
-          cudaDeviceGetDefaultMemPool(&pool, dev);
-          return pool;
-        }(), 0));
+      if (!p) {  // memory the pools hold may be returned to the device
+        trimPool();
         p = countedAlloc(bytes);
       }
       if (p) {
