@@ -741,27 +741,33 @@ std::string stagedKernels(int fnKind) {
   return fnKind == WS_JF_NOKEYS ? "WS_K_NOKEYS_STAGED(QEv, wsq)\n"
          : fnKind == WS_JF_DENSE ? "WS_K_DENSE_PRIV_STAGED(QEv, wsq)\n" : "";
 }
-// A plan's module: evaluators and kernels.  QHot's direct kernels have the prefix wsq.  QEv's are compiled too
-// (prefix wsg) when a column may be stored otherwise than hinted, i.e. when any hint is an encoding; without a
-// QHot they are the plan's only ones (prefix wsq).
+// A plan's sources.  `evaluators` (QEv, QHot) identify the plan.  With a QHot its direct kernels (prefix wsq) are compiled
+// when the plan is asked for; QEv's run batches stored otherwise than hinted (some hint is an encoding) and
+// are compiled at the first call with such a batch, staged kernels (QEv) at the first staged launch: compiling all of
+// them with the plan took 1.2 to 6 times as long (five aggregates over encoded columns 4.5 -> 19.7 s).  A plan without
+// GROUP BY has its QEv kernels at once: they are small, and the no-allocation entry cannot compile.
 struct PlanSource {
-  std::string evaluators, kernels;
+  std::string evaluators, main, any, staged;
   std::vector<std::pair<int, int>> encs;  // what QHot relies on
   bool hot = false;
   int stageBytes = 0, denseV = 1;  // QHot::DENSE_V
 };
 PlanSource planSource(const ws_expr_env& env, int ncols, const ws_agg_plan& plan, int fnKind) {
   PlanSource p;
-  p.evaluators = genEvaluator(env, ncols, plan, fnKind, &p.stageBytes);
+  const std::string ev = genEvaluator(env, ncols, plan, fnKind, &p.stageBytes);
   const std::string hot = genHot(env, ncols, plan, fnKind, &p.encs, &p.denseV);
   p.hot = !hot.empty();
-  p.evaluators += hot;
+  p.evaluators = ev + hot;
   bool hinted = false;
   for (auto& [c, e] : p.encs) hinted |= e != 0;
-  if (p.hot) p.kernels += directKernels(fnKind, "QHot", "wsq");
-  if (!p.hot) p.kernels += directKernels(fnKind, "QEv", "wsq");
-  else if (hinted) p.kernels += directKernels(fnKind, "QEv", "wsg");
-  p.kernels += stagedKernels(fnKind);
+  if (!p.hot) {
+    p.main = ev + directKernels(fnKind, "QEv", "wsq");
+  } else {
+    p.main = hot + directKernels(fnKind, "QHot", "wsq");
+    if (hinted) (fnKind == WS_JF_NOKEYS ? p.main : p.any) += ev + directKernels(fnKind, "QEv", "wsg");
+  }
+  const std::string staged = stagedKernels(fnKind);
+  if (!staged.empty() && p.stageBytes > 0) p.staged = ev + staged;
   return p;
 }
 
@@ -913,28 +919,47 @@ CUmodule compileModule(const std::string& body, bool* fromDisk) {
   return mod;
 }
 
-void compileProgram(ws_jit_program& p) {
-  const std::string body = p.source + p.kernelSource;
-  bool disk = false;
-  p.module = compileModule(body, &disk);
-  p.fromDisk = disk;
-  static const char* names[K_COUNT_] = {"nokeys", "dense_shared", "dense_global", "hash", "select", "dense_priv", "dense_priv_staged", "multi_nokeys", "multi_dense_priv",
-                                        "multi_hash", "nokeys_staged"};
-  auto find = [&](const std::string& name) {
-    CUfunction f = nullptr;
-    return drv().moduleGetFunction(&f, p.module, name.c_str()) == CUDA_SUCCESS ? f : nullptr;
-  };
+// The scan kernels of a module by their prefix.
+void findKernels(CUmodule m, const char* prefix, KernelSet& set) {
+  static const char* names[K_COUNT_] = {"nokeys", "dense_shared", "dense_global", "hash", "select", "dense_priv",
+                                        "dense_priv_staged", "multi_nokeys", "multi_dense_priv", "multi_hash",
+                                        "nokeys_staged"};
   for (int k = 0; k < K_COUNT_; ++k) {
-    p.kernels.fn[k] = find(std::string("wsq_") + names[k]);
-    p.generic.fn[k] = p.hot ? find(std::string("wsg_") + names[k]) : nullptr;
-    // a plan without encoded columns needs no other kernels, nor do the staged ones differ
-    if (!p.generic.fn[k]) {
-      p.generic.fn[k] = p.kernels.fn[k];
-      if (k == K_DENSE_SHARED) p.generic.denseV = p.kernels.denseV;
-    }
+    CUfunction f = nullptr;
+    if (drv().moduleGetFunction(&f, m, (std::string(prefix) + names[k]).c_str()) == CUDA_SUCCESS) set.fn[k] = f;
   }
-  p.kernels.interp = p.generic.interp = false;
+  set.interp = false;
 }
+
+void compileProgram(ws_jit_program& p) {
+  bool disk = false;
+  p.module = compileModule(p.mainSource, &disk);
+  p.fromDisk = disk;
+  findKernels(p.module, "wsq_", p.kernels);
+  if (p.hot && p.anySource.empty()) {  // nothing is hinted (QHot runs every batch), or wsg kernels are here too
+    findKernels(p.module, "wsg_", p.any);
+    for (int k = 0; k < K_COUNT_; ++k)
+      if (!p.any.fn[k]) p.any.fn[k] = p.kernels.fn[k], p.any.denseV = p.kernels.denseV;
+    p.anyState.store(1, std::memory_order_release);
+  }
+}
+
+// Compiles a module of p at its first use, once (state: see ws_jit_program).
+void compileLater(const ws_jit_program& p, const std::string& source, const char* prefix, KernelSet& set,
+                  std::atomic<int>& state) {
+  std::lock_guard<std::mutex> g(p.buildMu);
+  const int st = state.load(std::memory_order_acquire);
+  if (st == 1 || st == 2) return;
+  bool ok = false;
+  try {
+    findKernels(compileModule(source, nullptr), prefix, set);
+    ok = true;
+  } catch (const std::exception& e) {
+    fprintf(stderr, "[warpstore_b200] codegen failed: %s\n", e.what());
+  }
+  state.store(ok ? 1 : 2, std::memory_order_release);
+}
+void compileAny(const ws_jit_program& p) { compileLater(p, p.anySource, "wsg_", p.any, p.anyState); }
 
 void compileAndPublish(const std::shared_ptr<ws_jit_program>& p) {
   auto t0 = std::chrono::steady_clock::now();
@@ -954,6 +979,21 @@ void compileAndPublish(const std::shared_ptr<ws_jit_program>& p) {
 }  // namespace ws
 
 using namespace ws;
+
+const KernelSet* ws_jit_program::anyStorage(bool wait) const {
+  int st = anyState.load(std::memory_order_acquire);
+  if (st == 0 && !wait && !sync && anyState.compare_exchange_strong(st, 3)) {
+    std::shared_ptr<const ws_jit_program> p = shared_from_this();
+    std::thread([p] { compileAny(*p); }).detach();
+  }
+  if (wait || sync) compileAny(*this);
+  return anyState.load(std::memory_order_acquire) == 1 ? &any : nullptr;
+}
+CUfunction ws_jit_program::stagedKernel(KernelId k) const {
+  if (stagedSource.empty()) return nullptr;
+  compileLater(*this, stagedSource, "wsq_", staged, stagedState);
+  return staged.fn[k];
+}
 
 extern "C" {
 
@@ -1017,7 +1057,9 @@ int ws_jit_get(const ws_expr_env* env, int ncols, const ws_agg_plan* plan, int f
         p->kind = kind ? kind : "";
         p->sql = tSql;
         p->source = ev;
-        p->kernelSource = src.kernels;
+        p->mainSource = src.main;
+        p->anySource = src.any;
+        p->stagedSource = src.staged;
         p->hot = src.hot;
         if (src.hot) p->kernels.denseV = src.denseV;
         p->encs = src.encs;
@@ -1029,6 +1071,7 @@ int ws_jit_get(const ws_expr_env* env, int ncols, const ws_agg_plan* plan, int f
       if (gByShape.size() >= kMaxShapes) gByShape.clear();
       gByShape[shape] = p;
     }
+    if (mode == WS_JIT_SYNC) p->sync = true;
     if (fresh) {
       if (mode == WS_JIT_SYNC) {
         compileAndPublish(p);
@@ -1038,7 +1081,10 @@ int ws_jit_get(const ws_expr_env* env, int ncols, const ws_agg_plan* plan, int f
           tInfo.compile_ms += p->compileMs;
         }
       } else {
-        std::thread([p] { compileAndPublish(p); }).detach();  // run interpreted now, compiled next time
+        std::thread([p] {  // run interpreted now, compiled next time
+          compileAndPublish(p);
+          if (p->state.load() == 1 && !p->anySource.empty()) compileAny(*p);
+        }).detach();
       }
     } else if (mode == WS_JIT_SYNC) {
       for (int spins = 0; p->state.load(std::memory_order_acquire) == 0; ++spins)  // compiled by another thread
@@ -1072,8 +1118,7 @@ int ws_codegen_source(const ws_expr_env* env, int ncols, const ws_agg_plan* plan
 int ws_codegen_compile_check(const ws_expr_env* env, int ncols, const ws_agg_plan* plan, int fn, int arch_sm,
                              size_t* cubin_bytes) {
   return guardedCall([&] {
-    const PlanSource src = planSource(*env, ncols, *plan, fn);
-    const std::string body = src.evaluators + src.kernels;
+    const std::string body = planSource(*env, ncols, *plan, fn).main;
     const std::string image = nvrtcCubin("#include \"ws_kern.cuh\"\n" + body, archOpts(arch_sm));
     if (cubin_bytes) *cubin_bytes = image.size();
   });

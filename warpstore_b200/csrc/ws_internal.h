@@ -175,28 +175,37 @@ unsigned persistentGrid(CUfunction f, size_t smem, int64_t ntiles, int threads =
 
 // A compiled plan (the engine's JitProgram, src/jit.h:16-31): generated evaluator source, its module
 // and kernels, state and statistics.
-struct ws_jit_program {
+struct ws_jit_program : std::enable_shared_from_this<ws_jit_program> {
   int id = 0;
   int fnKind = 0;
   std::string kind, sql, source;
-  std::string kernelSource;  // kernel instantiations compiled after `source`
+  // The module compiled when a plan is asked for (every direct-load kernel of its evaluator), and those compiled at the
+  // first call that needs them: kernels for batches stored otherwise than hinted, and staged kernels ("": none).
+  std::string mainSource, anySource, stagedSource;
   // hot: `kernels` are instantiated with the evaluator of hinted storage, which only runs batches whose columns
-  // are stored as `encs` (column, encoding) says; `generic` runs any batch the plan covers.
+  // are stored as `encs` (column, encoding) says; `any` runs any batch the plan covers.
   bool hot = false;
   std::vector<std::pair<int, int>> encs;
   double compileMs = 0;
   std::atomic<int> state{0};  // 0 compiling, 1 ready, 2 failed
   bool fromDisk = false;
   int stageBytes = 0;  // shared memory per staged tile (0: the plan reads global memory directly)
-  ws::KernelSet kernels, generic;
-  // The kernels that can run these batches.
-  const ws::KernelSet& kernelsFor(int nb, int ncols, const ws_col_view* bcols) const {
-    if (!hot) return kernels;
+  ws::KernelSet kernels;
+  mutable ws::KernelSet any, staged;                         // filled by anyStorage / stagedKernel
+  mutable std::atomic<int> anyState{0}, stagedState{0};      // 0 not compiled, 1 ready, 2 failed, 3 compiling (another thread)
+  mutable std::mutex buildMu;                                // held while one of them is compiled
+  std::atomic<bool> sync{false};  // asked for in WS_JIT_SYNC: its later modules are waited for too
+  // The kernels that can run these batches; null: not compiled yet, and the caller (wait false) interprets the
+  // plan meanwhile, as it does while the plan itself is compiled.
+  const ws::KernelSet* kernelsFor(int nb, int ncols, const ws_col_view* bcols, bool wait) const {
+    if (!hot) return &kernels;
     for (int b = 0; b < nb; ++b)
       for (auto& [c, e] : encs)
-        if (bcols[(int64_t)b * ncols + c].enc != e) return generic;
-    return kernels;
+        if (bcols[(int64_t)b * ncols + c].enc != e) return anyStorage(wait);
+    return &kernels;
   }
+  const ws::KernelSet* anyStorage(bool wait) const;
+  CUfunction stagedKernel(ws::KernelId k) const;  // compiled when first asked for; null: none
   CUmodule module = nullptr;
   std::mutex mu;
   int64_t execs = 0;

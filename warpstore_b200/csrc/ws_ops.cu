@@ -624,8 +624,12 @@ static void aggRun(ws_aggregator& A, const ws_expr_env& env, const ws_jit_progra
   const int nb = (int)A.bn.size();
   if (nb == 0) return;
   A.newRun();
-  const bool useJit = jit && jit->state.load() == 1 && planCovers(env, nb, A.ncols, A.bcols.data());
-  if (!useJit && (A.plan.naggs > WS_INTERP_AGGS || A.plan.nkeys > WS_INTERP_KEYS))
+  const bool interpretable = A.plan.naggs <= WS_INTERP_AGGS && A.plan.nkeys <= WS_INTERP_KEYS;
+  // a prepared query keeps the kernel it gets, and a plan the interpreter cannot run has no other: both wait for it
+  const KernelSet* compiled = jit && jit->state.load() == 1 && planCovers(env, nb, A.ncols, A.bcols.data())
+                                  ? jit->kernelsFor(nb, A.ncols, A.bcols.data(), prep || !interpretable) : nullptr;
+  const bool useJit = compiled != nullptr;
+  if (!useJit && !interpretable)
     throw Error("this aggregation needs a compiled plan (more than 16 aggregates or 4 GROUP BY keys); codegen failed or is off", WS_ERR_PLAN);
   std::unique_ptr<TProgs> progs;
   if (!useJit) {
@@ -639,8 +643,7 @@ static void aggRun(ws_aggregator& A, const ws_expr_env& env, const ws_jit_progra
   L.rows = A.rows.p;
   L.err = A.err();
   L.ticket = A.ticket();
-  const KernelSet& ks = useJit ? jit->kernelsFor(nb, A.ncols, A.bcols.data()) : interpKernels();
-  const KernelSet& anyStorage = useJit ? jit->generic : ks;  // staged kernels
+  const KernelSet& ks = useJit ? *compiled : interpKernels();
   // Staged scans: a ring of 2..4 tile stages in shared memory (compiled plans only).
   const int stageBytes = useJit ? jit->stageBytes : 0;
   static const int maxStages = [] {  // WARPSTORE_B200_STAGES: shared-memory tile stages (0: direct loads,
@@ -674,13 +677,14 @@ static void aggRun(ws_aggregator& A, const ws_expr_env& env, const ws_jit_progra
   };
   Launch* lp = &L;
   if (A.plan.nkeys == 0) {
-    CUfunction f = ks.fn[K_NOKEYS], stagedFn = anyStorage.fn[K_NOKEYS_STAGED];
+    CUfunction f = ks.fn[K_NOKEYS];
     if (!f) throw Error("compiled plan has no aggregation kernel", WS_ERR_INTERNAL);
     shapeOf = [=](const TuneChoice& c) {
       // stage count: the choice's, else the default; within 200 KB of tile stages
       int st = c.stages >= 0 ? c.stages : S;
       if (stageBytes > 0) st = (int)std::min<int64_t>(st, (200 * 1024) / stageBytes);
-      if (st < 2 || stageBytes <= 0 || !stagedFn) st = 0;
+      CUfunction stagedFn = st < 2 || stageBytes <= 0 ? nullptr : jit->stagedKernel(K_NOKEYS_STAGED);
+      if (!stagedFn) st = 0;
       lp->stages = st;
       return Shape{st ? stagedFn : f, (size_t)st * stageBytes, st ? kStagedThreads : kThreads};
     };
@@ -720,17 +724,18 @@ static void aggRun(ws_aggregator& A, const ws_expr_env& env, const ws_jit_progra
       // tile stages fit beside the private rows within 220 KB; the staged body is its own entry
       const int64_t room = std::max<int64_t>(0, (int64_t)(220 * 1024) - (int64_t)privBytes);
       const int fitStages = stageBytes > 0 ? (int)std::min<int64_t>(8, room / stageBytes) : 0;
-      CUfunction direct = ks.fn[K_DENSE_PRIV], stagedFn = anyStorage.fn[K_DENSE_PRIV_STAGED];
+      CUfunction direct = ks.fn[K_DENSE_PRIV];
       shapeOf = [=](const TuneChoice& c) {
         int st = std::min(c.stages >= 0 ? c.stages : maxStages, fitStages);
-        if (st < 2 || !stagedFn) st = 0;
+        CUfunction stagedFn = st < 2 ? nullptr : jit->stagedKernel(K_DENSE_PRIV_STAGED);
+        if (!stagedFn) st = 0;
         lp->stages = st;
         return Shape{st ? stagedFn : direct, (size_t)st * stageBytes + privBytes, st ? kStagedThreads : kThreads};
       };
       name = "dense_priv";
       partRows = G;
       cands.push_back(ctas(1));
-      if (stagedFn && fitStages >= 2)
+      if (fitStages >= 2)
         for (int st : {0, 2, 3})
           if (st <= fitStages && st != (std::min(maxStages, fitStages) >= 2 ? std::min(maxStages, fitStages) : 0))
             cands.push_back(staged(st));
@@ -1003,8 +1008,8 @@ static MultiPlan planMulti(const std::vector<const PreparedScan*>& preps, const 
     const PreparedScan& p = *preps[i];
     if (!p.ready) continue;  // no tiles: nothing to scan
     if (p.compiled && !jit) throw Error(std::string(who) + ": compiled queries need their plan", WS_ERR_ARG);
-    const KernelSet& own = !p.compiled ? interpKernels() : p.hot ? jit->kernels : jit->generic;
-    const KernelSet& k = !p.compiled ? interpKernels() : hot ? jit->kernels : jit->generic;
+    const KernelSet& own = !p.compiled ? interpKernels() : p.hot ? jit->kernels : jit->any;
+    const KernelSet& k = !p.compiled ? interpKernels() : hot ? jit->kernels : jit->any;
     const int m = p.scan < 0 || p.f != own.fn[p.scan] ? -1
                 : p.scan == K_NOKEYS ? K_MULTI_NOKEYS : p.scan == K_DENSE_PRIV ? K_MULTI_DENSE_PRIV : K_MULTI_HASH;
     if (m < 0 || !k.fn[m] || p.L.stages)

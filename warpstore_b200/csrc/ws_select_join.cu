@@ -761,14 +761,15 @@ static int64_t selectRun(const ws_expr_env& env, bool hasWhere, ws_prog where, i
   fp.where = where;
   fp.naggs = 1;
   fp.ops[0] = WS_AGG_COUNT;
-  const bool useJit = jit && jit->state.load() == 1 && jit->kernels.fn[K_SELECT] && [&] {
+  const bool covered = jit && jit->state.load() == 1 && jit->kernels.fn[K_SELECT] && [&] {
     for (int b = 0; b < nb; ++b)
       for (int c = 0; c < ncols; ++c)
         if (bcols[(int64_t)b * ncols + c].enc && !env.cols[c].enc) return false;
     return true;
   }();
+  const KernelSet* compiled = covered ? jit->kernelsFor(nb, ncols, bcols, false) : nullptr;
   std::unique_ptr<TProgs> progs;
-  if (!useJit) {
+  if (!compiled) {
     progs.reset(new TProgs);
     buildTProgs(env, ncols, fp, hasWhere, *progs);
   }
@@ -787,7 +788,7 @@ static int64_t selectRun(const ws_expr_env& env, bool hasWhere, ws_prog where, i
   L.progs = d.progs;
   L.naggs = 1;
   L.rowWords = 1;
-  const KernelSet& ks = useJit ? jit->kernelsFor(nb, ncols, bcols) : interpKernels();
+  const KernelSet& ks = compiled ? *compiled : interpKernels();
   DBuf<int64_t> counts(d.ntiles + 1);
   L.tileCount = (i64*)counts.p;
   DBuf<uint32_t> mask(d.ntiles * (kTile / 32));
