@@ -988,52 +988,69 @@ WS_DI u64 globalPeek(const Launch& L, const Ev& ev, u64 kw) {
 template <class Ev>
 WS_DI void globalInsert(const Launch& L, const Ev& ev, u64 kw, const double* kv, const u64* x, u64 first) {
   const int rw = ev.rowWords();
+  // The probe loop only finds the row: the lanes of a warp find theirs after different numbers of steps, and add
+  // together behind it.  Every kProbeRound steps they meet, so that a lane that raised the overflow flag has stored it before
+  // the others probe on (else the warp may run its longest probe, of up to probeLimit steps, first), and those stop
+  // there once the table has overflowed.
+  constexpr int kProbeRound = 64;
+  u64* hit = nullptr;
   if (kw == kEmpty) {  // the EMPTY key word itself has a dedicated row after the table (a single key: it is the key)
-    u64* row = L.table + (L.mask + 1) * rw;
-    if (atomicCAS(row, 0ull, 1ull) == 0ull && ev.nk() > 1)
+    hit = L.table + (L.mask + 1) * rw;
+    if (atomicCAS(hit, 0ull, 1ull) == 0ull && ev.nk() > 1)
       for (int k = 0; k < ev.nk(); ++k) L.tkeys[(L.mask + 1) * ev.nk() + k] = kv[k];
-    rowAtomicCombine(ev, row, x);
-    return;
   }
+  const unsigned lanes = __activemask();
   u64 s = mix64(kw) & L.mask;
-  for (int p = 0; p < L.probeLimit; ++p) {
-    u64* row = L.table + s * rw;
-    u64 prev = p ? *(volatile u64*)row : first;
-    if (prev == kEmpty) {
-      prev = atomicCAS(row, kEmpty, kw);
+  for (int p0 = 0;; p0 += kProbeRound) {
+    const int end = hit ? p0 : min(p0 + kProbeRound, L.probeLimit);
+#pragma unroll 1
+    for (int p = p0; p < end; ++p) {
+      u64* row = L.table + s * rw;
+      u64 prev = p ? *(volatile u64*)row : first;
       if (prev == kEmpty) {
-        if (ev.nk() > 1)
-          for (int k = 0; k < ev.nk(); ++k) L.tkeys[s * ev.nk() + k] = kv[k];
-        const u64 c = atomicAdd(L.count, 1ull) + 1;
-        if (c * 10 > (L.mask + 1) * 7) L.err[1] = 1;  // fuller than 70%: the caller retries bigger
-        prev = kw;
+        prev = atomicCAS(row, kEmpty, kw);
+        if (prev == kEmpty) {
+          if (ev.nk() > 1)
+            for (int k = 0; k < ev.nk(); ++k) L.tkeys[s * ev.nk() + k] = kv[k];
+          const u64 c = atomicAdd(L.count, 1ull) + 1;
+          if (c * 10 > (L.mask + 1) * 7) *(volatile int*)(L.err + 1) = 1;  // fuller than 70%: the caller retries bigger
+          prev = kw;
+        }
       }
+      if (prev == kw) {
+        hit = row;
+        break;
+      }
+      s = (s + 1) & L.mask;
     }
-    if (prev == kw) {
-      rowAtomicCombine(ev, row, x);
-      return;
-    }
-    s = (s + 1) & L.mask;
+    __syncwarp(lanes);
+    const bool more = !hit && end < L.probeLimit && !*(volatile int*)(L.err + 1);
+    if (!__any_sync(lanes, more)) break;
   }
-  L.err[1] = 1;  // no free slot within the probe limit
+  if (hit) rowAtomicCombine(ev, hit, x);
+  else *(volatile int*)(L.err + 1) = 1;  // no free slot within the probe limit
 }
 
 // A list of n rows into the global table, Ev::FLUSH_ROWS per thread at a time: key(j) is row j's key word (kEmpty:
-// no first probe), insert(j, key word, first) inserts it.
+// no first probe), insert(j, key word, first) inserts it.  A thread stops once the table has overflowed (the run's
+// result is discarded then); the flag is read beside the first probes, so it adds no wait.
 template <class Ev, class Key, class Insert>
 WS_DI void insertAll(const Launch& L, const Ev& ev, int n, Key&& key, Insert&& insert) {
   for (int j0 = threadIdx.x; j0 < n; j0 += blockDim.x * Ev::FLUSH_ROWS) {
     u64 kw[Ev::FLUSH_ROWS], first[Ev::FLUSH_ROWS];
+    const int overflowed = *(volatile int*)(L.err + 1);
 #pragma unroll
     for (int r = 0; r < Ev::FLUSH_ROWS; ++r) {
       const int j = j0 + r * (int)blockDim.x;
       kw[r] = j < n ? key(j) : kEmpty;
       first[r] = kw[r] != kEmpty ? globalPeek(L, ev, kw[r]) : 0ull;
     }
+    if (overflowed) return;
+#pragma unroll 1
+    for (int j = j0, r = 0; r < Ev::FLUSH_ROWS && j < n; ++r, j += blockDim.x) {
+      insert(j, kw[0], first[0]);
 #pragma unroll
-    for (int r = 0; r < Ev::FLUSH_ROWS; ++r) {
-      const int j = j0 + r * (int)blockDim.x;
-      if (j < n) insert(j, kw[r], first[r]);
+      for (int q = 0; q + 1 < Ev::FLUSH_ROWS; ++q) kw[q] = kw[q + 1], first[q] = first[q + 1];
     }
   }
 }
@@ -1130,10 +1147,10 @@ __device__ void aggHash(const Launch& L) {
       globalInsert(L, ev, kw, kv, x, globalPeek(L, ev, kw));
     }
   };
-  // Inserts the buffered rows (force: however few); returns true (in every thread) once the global table has
-  // overflowed: the run's result is discarded then (the caller reruns with a bigger table), so the CTA stops.
-  auto flush = [&](bool force) -> bool {
-    if (!__syncthreads_or(appended || force)) return false;
+  // Inserts the buffered rows; returns true (in every thread) once the global table has overflowed: the run's result is
+  // discarded then (the caller reruns with a bigger table), so the CTA stops.
+  auto flush = [&]() -> bool {
+    if (!__syncthreads_or(appended)) return false;
     // every thread is past its appends and none appends before the last barrier below
     const int n = min(spillN, B);
     if (threadIdx.x == 0) stopFlag = *(volatile int*)(L.err + 1);
@@ -1153,8 +1170,8 @@ __device__ void aggHash(const Launch& L) {
     __syncthreads();  // the buffer is refilled by the next tile
     return false;
   };
-  forEachRowTiles(L, ev, rowFn, [&]() { return flush(false); });
-  if (flush(true)) return;  // overflowed: the shared table is not merged either
+  forEachRowTiles(L, ev, rowFn, flush);
+  __syncthreads();  // every tile ended with a flush: only the shared table is left (an overflowed run merges nothing)
   insertAll(
       L, ev, S, [&](int s) { return tkey[s]; },
       [&](int s, u64 kw, u64 first) {

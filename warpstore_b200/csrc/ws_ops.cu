@@ -65,7 +65,9 @@ struct FillSpec {
   u64* ctl;            // kCtlWords words
   RowTemplate t;
 };
-constexpr int kCtlWords = 4;
+// count u64 | ... | err int x3, occTicket u32 | ticket u32, pad: the flags that scans read are 128 bytes from the count
+// that they add to, so that those reads do not queue behind its atomics.
+constexpr int kCtlWords = 24, kCtlFlags = 128;
 // Thread `tid` of `nthreads` (at least rw).  The threads step by a multiple of the row width, so each stays
 // on one word of the rows (a constant) and a warp's stores are consecutive: 2^24 rows of 32 B take 79 us,
 // against 310 us with a row per thread (and 345 us with a loop of its own for the key words).
@@ -487,7 +489,7 @@ struct ws_aggregator {
   int batchesDone = 0, windows = 0;
   DBuf<u64> rows;
   DBuf<double> tkeys;
-  // control words (kCtlWords u64 after the rows): [count u64][err int x3][occTicket u32][ticket u32][pad]
+  // control words after the rows (kCtlWords)
   uint8_t* ctl() { return (uint8_t*)(rows.p + nrows() * lay.rw); }
   std::vector<int64_t> hi;
   // What the last fetch learned of the run's result, until the next run: the status (flags, groups), of a small
@@ -501,9 +503,9 @@ struct ws_aggregator {
   void newRun() { statusKnown = groupsOnHost = offsKnown = false; }
 
   u64* count() { return (u64*)ctl(); }
-  int* err() { return (int*)(ctl() + 8); }
-  unsigned* occTicket() { return (unsigned*)(ctl() + 20); }
-  unsigned* ticket() { return (unsigned*)(ctl() + 24); }
+  int* err() { return (int*)(ctl() + kCtlFlags); }
+  unsigned* occTicket() { return (unsigned*)(ctl() + kCtlFlags + 12); }
+  unsigned* ticket() { return (unsigned*)(ctl() + kCtlFlags + 16); }
   int64_t nrows() const { return isDense ? dense.G : plan.nkeys ? cap + 1 : 1; }
 };
 
