@@ -733,7 +733,7 @@ std::string directKernels(int fnKind, const std::string& ev, const std::string& 
     case WS_JF_NOKEYS: return "WS_K_NOKEYS" + a + "WS_K_MULTI_NOKEYS" + a;
     case WS_JF_GROUPED: return "WS_K_HASH" + a + "WS_K_MULTI_HASH" + a;
     case WS_JF_DENSE:
-      return "WS_K_DENSE_PRIV" + a + "WS_K_DENSE_SHARED" + a + "WS_K_DENSE_GLOBAL" + a + "WS_K_MULTI_DENSE_PRIV" + a;
+      return "WS_K_DENSE_PRIV" + a + "WS_K_DENSE_SHARED" + a + "WS_K_DENSE_TOPS" + a + "WS_K_DENSE_GLOBAL" + a + "WS_K_MULTI_DENSE_PRIV" + a;
     default: return "WS_K_SELECT" + a;
   }
 }
@@ -923,7 +923,7 @@ CUmodule compileModule(const std::string& body, bool* fromDisk) {
 void findKernels(CUmodule m, const char* prefix, KernelSet& set) {
   static const char* names[K_COUNT_] = {"nokeys", "dense_shared", "dense_global", "hash", "select", "dense_priv",
                                         "dense_priv_staged", "multi_nokeys", "multi_dense_priv", "multi_hash",
-                                        "nokeys_staged"};
+                                        "nokeys_staged", "dense_tops"};
   for (int k = 0; k < K_COUNT_; ++k) {
     CUfunction f = nullptr;
     if (drv().moduleGetFunction(&f, m, (std::string(prefix) + names[k]).c_str()) == CUDA_SUCCESS) set.fn[k] = f;

@@ -152,11 +152,11 @@ EnvK envK(const ws_expr_env& env);
 // K_DENSE_PRIV_STAGED, K_NOKEYS_STAGED: the same bodies with a producer warp staging tiles by TMA (kStagedThreads).
 enum KernelId {
   K_NOKEYS = 0, K_DENSE_SHARED, K_DENSE_GLOBAL, K_HASH, K_SELECT, K_DENSE_PRIV,
-  K_DENSE_PRIV_STAGED, K_MULTI_NOKEYS, K_MULTI_DENSE_PRIV, K_MULTI_HASH, K_NOKEYS_STAGED, K_COUNT_
+  K_DENSE_PRIV_STAGED, K_MULTI_NOKEYS, K_MULTI_DENSE_PRIV, K_MULTI_HASH, K_NOKEYS_STAGED, K_DENSE_TOPS, K_COUNT_
 };
 struct KernelSet {
   CUfunction fn[K_COUNT_] = {};
-  int denseV = 1;  // K_DENSE_SHARED's CTA: denseV * kThreads threads
+  int denseV = 1;  // K_DENSE_SHARED's and K_DENSE_TOPS' CTA: denseV * kThreads threads
   bool interp = true;
 };
 const KernelSet& interpKernels();

@@ -766,19 +766,21 @@ __device__ void aggDensePriv(const Launch& L) {
 }
 
 // ------------------------------------------------------------------ compact accumulators
-// A group's accumulators in a CTA's shared-memory table: a 64-bit word per slot (COUNT: 32 bits, in an array of
-// their own), updated by 32-bit shared atomics where a 64-bit one would be a compare-and-swap loop:
+// A group's accumulators in a CTA's shared-memory table: a 64-bit word per slot (COUNT: none) and 32-bit words in arrays
+// of their own (COUNT: its count; integer SUM: the bits above the word's 64), updated by 32-bit shared atomics where a
+// 64-bit one would be a compare-and-swap loop:
 //   COUNT   one 32-bit addition (a CTA visits fewer than 2^32 rows);
-//   integer SUM   the low half added with its old value returned, the high half and the carry only when that sum
-//           is not zero, i.e. rarely for small non-negative arguments.  The word is exact modulo 2^64 and must not leave the
-//           int64 range: a row whose arguments break the bound of sumMagnitude for the whole CTA's rows
-//           (compactOk) does not go through the table;
+//   integer SUM   a 96-bit number in three words: the low word added with its old value returned, the middle word and
+//           the carry only when their sum is not zero, i.e. rarely for small arguments, the top word only when the
+//           middle addition's carry does not cancel the argument's sign.  2^32 rows of any int64 fit 96 bits, so the
+//           sum is exact for every argument (COUNT and two SUMs into 16 groups, 8M rows: 75 us, arguments of 2^51 78 us;
+//           those took 3730 us when words of 64 bits sent them to the global table);
 //   MIN / MAX   a read, and an atomic only when the row improves on it;
 //   DOUBLE SUM   a 64-bit atomic.
 // A table of E entries holds each slot's words together (word o64 of entry e at t64[o64 * E + e]): the lanes of a warp
 // update one slot of random entries at a time, which then spread over all banks (words entry by entry, four to an
 // entry, met in 4 bank pairs, 98 shared-memory wavefronts per 32 rows of five aggregates: 168 us where this takes 118).
-// Against accumulator rows of 64-bit and 128-bit words: 36 instead of 56 bytes for COUNT, SUM, MIN, MAX and a DOUBLE
+// Against accumulator rows of 64-bit and 128-bit words: 40 instead of 56 bytes for COUNT, SUM, MIN, MAX and a DOUBLE
 // SUM, so the table takes more groups or leaves room for more warps.
 //
 // The interpreter (COMPACT = false) keeps whole accumulator rows there, entry by entry: its slots' kinds and offsets are
@@ -787,7 +789,7 @@ __device__ void aggDensePriv(const Launch& L) {
 //
 // t64 / t32: the table's words, E entries; e: an entry; x: a row's accumulator words (rowOfInput).
 template <class Ev>
-WS_DI void compactWords(const Ev& ev, int& n64, int& n32) {
+WS_DI void compactWords(const Ev& ev, bool tops, int& n64, int& n32) {
   n64 = n32 = 0;
   if constexpr (!Ev::COMPACT) {
     n64 = ev.rowWords();
@@ -795,17 +797,24 @@ WS_DI void compactWords(const Ev& ev, int& n64, int& n32) {
 #pragma unroll
     for (int a = 0; a < Ev::NA; ++a) {
       const int k = ev.kind(a);
-      n32 += k == SK_COUNT;
+      n32 += k == SK_COUNT || (k == SK_ISUM && tops);
       n64 += k != SK_COUNT && k != SK_NONE;
     }
   }
 }
 template <class Ev>
-WS_DI void compactIdentity(const Ev& ev, u64* t64, unsigned* t32, unsigned e, unsigned E) {
+WS_DI unsigned compactTop0(const Ev& ev) {  // the top words' arrays start behind the counts'
+  unsigned n = 0;
+#pragma unroll
+  for (int a = 0; a < Ev::NA; ++a) n += ev.kind(a) == SK_COUNT;
+  return n;
+}
+template <class Ev>
+WS_DI void compactIdentity(const Ev& ev, bool tops, u64* t64, unsigned* t32, unsigned e, unsigned E) {
   if constexpr (!Ev::COMPACT) {
     rowIdentity(ev, t64 + (size_t)e * ev.rowWords());
   } else {
-    unsigned o64 = e, o32 = e;
+    unsigned o64 = e, o32 = e, oTop = e + compactTop0(ev) * E;
 #pragma unroll
     for (int a = 0; a < Ev::NA; ++a) {
       const int k = ev.kind(a);
@@ -816,12 +825,16 @@ WS_DI void compactIdentity(const Ev& ev, u64* t64, unsigned* t32, unsigned e, un
         u64 hi;
         slotIdentity(k, t64[o64], hi);
         o64 += E;
+        if (k == SK_ISUM) {
+          if (tops) t32[oTop] = 0;
+          oTop += E;
+        }
       }
     }
   }
 }
-// Row i (words x) may be added to compact words: the sums of all the CTA's rows (2^8 threads of at most
-// 2^(31 - sumShift) rows each) stay in the int64 range.
+// A row (words x) may be added to compact words without top words: the sums of all the CTA's rows (2^8 threads of at
+// most 2^(31 - sumShift) rows each) stay in the int64 range.
 template <class Ev>
 WS_DI bool compactOk(const Launch& L, const Ev& ev, const u64* x, int i) {
   if constexpr (!Ev::COMPACT) return true;
@@ -836,11 +849,11 @@ WS_DI bool compactOk(const Launch& L, const Ev& ev, const u64* x, int i) {
   return L.sumShift >= 8 && (m >> (L.sumShift - 8)) == 0;
 }
 template <class Ev>
-WS_DI void compactAdd(const Ev& ev, const u64* x, u64* t64, unsigned* t32, unsigned e, unsigned E) {
+WS_DI void compactAdd(const Ev& ev, bool tops, const u64* x, u64* t64, unsigned* t32, unsigned e, unsigned E) {
   if constexpr (!Ev::COMPACT) {
     rowAtomicCombine(ev, t64 + (size_t)e * ev.rowWords(), x);
   } else {
-    unsigned o64 = e, o32 = e;
+    unsigned o64 = e, o32 = e, oTop = e + compactTop0(ev) * E;
 #pragma unroll
     for (int a = 0; a < Ev::NA; ++a) {
       const int k = ev.kind(a);
@@ -857,8 +870,15 @@ WS_DI void compactAdd(const Ev& ev, const u64* x, u64* t64, unsigned* t32, unsig
         case SK_ISUM: {
           const unsigned lo = (unsigned)v;
           unsigned h = (unsigned)(v >> 32);
-          if (lo) h += atomicAdd((unsigned*)p, lo) + lo < lo;  // the carry of the low half
-          if (h) atomicAdd((unsigned*)p + 1, h);
+          if (lo) h += atomicAdd((unsigned*)p, lo) + lo < lo;  // the carry of the low word
+          if (h) {  // 0: nothing to add, or -1 and a carry, which leave the upper words as they are
+            const unsigned mid = atomicAdd((unsigned*)p + 1, h) + h;
+            if (tops) {
+              const int top = ((int)(v >> 32) >> 31) + (int)(mid < h);
+              if (top) atomicAdd(t32 + oTop, (unsigned)top);
+            }
+          }
+          oTop += E;
           break;
         }
         case SK_IMIN: case SK_DMIN: if ((i64)v < *(volatile i64*)p) atomicMin((i64*)p, (i64)v); break;
@@ -875,11 +895,11 @@ WS_DI void compactAdd(const Ev& ev, const u64* x, u64* t64, unsigned* t32, unsig
 }
 // w (an accumulator row) += entry e
 template <class Ev>
-WS_DI void compactInto(const Ev& ev, u64* w, const u64* t64, const unsigned* t32, unsigned e, unsigned E) {
+WS_DI void compactInto(const Ev& ev, bool tops, u64* w, const u64* t64, const unsigned* t32, unsigned e, unsigned E) {
   if constexpr (!Ev::COMPACT) {
     rowCombine(ev, w, t64 + (size_t)e * ev.rowWords());
   } else {
-    unsigned o64 = e, o32 = e;
+    unsigned o64 = e, o32 = e, oTop = e + compactTop0(ev) * E;
 #pragma unroll
     for (int a = 0; a < Ev::NA; ++a) {
       const int k = ev.kind(a), o = ev.woff(a);
@@ -890,7 +910,9 @@ WS_DI void compactInto(const Ev& ev, u64* w, const u64* t64, const unsigned* t32
         const u64 v = t64[o64];
         o64 += E;
         u64 one = 0;
-        slotCombine(k, w[o], k == SK_ISUM ? w[o + 1] : one, v, (u64)((i64)v >> 63));
+        slotCombine(k, w[o], k == SK_ISUM ? w[o + 1] : one, v,
+                    (u64)(k == SK_ISUM && tops ? (i64)(int)t32[oTop] : (i64)v >> 63));
+        if (k == SK_ISUM) oTop += E;
       }
     }
   }
@@ -903,16 +925,16 @@ WS_DI void compactInto(const Ev& ev, u64* w, const u64* t64, const unsigned* t32
 // rows into 1500 groups with five aggregates 215 -> 118 us (accumulator rows of 56 B and CTAs of 256 threads left 16
 // warps per SM), 12M into 5000 groups 377 -> 83 us (those rows did not fit, every row went to L2 atomics).  What bounds
 // it now is the shared-memory pipe (88 % busy): the atomics of random entries.
-template <class Ev>
+template <class Ev, bool tops>
 __device__ void aggDenseShared(const Launch& L) {
   extern __shared__ __align__(16) u64 wsSmem[];
   Ev ev(L);
   const int rw = ev.rowWords(), G = (int)L.G, C = L.copies, E = G * C;
   int n64, n32;
-  compactWords(ev, n64, n32);
+  compactWords(ev, tops, n64, n32);
   u64* t64 = wsSmem;
   unsigned* t32 = (unsigned*)(t64 + (size_t)E * n64);
-  for (int e = threadIdx.x; e < E; e += blockDim.x) compactIdentity(ev, t64, t32, e, E);
+  for (int e = threadIdx.x; e < E; e += blockDim.x) compactIdentity(ev, tops, t64, t32, e, E);
   __syncthreads();
   const int copy = threadIdx.x & (C - 1);
   forEachRow<Ev::DENSE_V>(L, ev, [&](int i, int, i64) {
@@ -921,20 +943,16 @@ __device__ void aggDenseShared(const Launch& L) {
       L.err[0] = 1;
       return;
     }
-    u64 x[kMaxRowWords];
+    u64 x[Ev::RW];
     rowOfInput(ev, i, x);
-    if (compactOk(L, ev, x, i)) {
-      const int e = (int)gi * C + copy;
-      compactAdd(ev, x, t64, t32, e, E);
-    } else {
-      rowAtomicCombine(ev, L.rows + gi * rw, x);
-    }
+    if (tops || compactOk(L, ev, x, i)) compactAdd(ev, tops, x, t64, t32, (int)gi * C + copy, E);
+    else rowAtomicCombine(ev, L.rows + gi * rw, x);
   });
   __syncthreads();
   for (int g = threadIdx.x; g < G; g += blockDim.x) {
-    u64 w[kMaxRowWords];
+    u64 w[Ev::RW];
     rowIdentity(ev, w);
-    for (int c = 0; c < C; ++c) compactInto(ev, w, t64, t32, g * C + c, E);
+    for (int c = 0; c < C; ++c) compactInto(ev, tops, w, t64, t32, g * C + c, E);
     if (w[ev.woff(0)] == 0) continue;  // slot 0 is COUNT(*): no rows of this group in this CTA
     rowAtomicCombine(ev, L.rows + (i64)g * rw, w);
   }
@@ -1056,8 +1074,7 @@ WS_DI void insertAll(const Launch& L, const Ev& ev, int n, Key&& key, Insert&& i
 }
 
 // Rows are pre-aggregated in a per-CTA shared-memory table (smemSlots key words with compact accumulators,
-// bounded probing), which absorbs hot keys.  A row that finds no slot there (or whose sums exceed the compact
-// bound) is appended to a per-CTA shared buffer (one shared atomic per warp); after a tile that appended any, the
+// bounded probing), which absorbs hot keys.  A row that finds no slot there is appended to a per-CTA shared buffer (one shared atomic per warp); after a tile that appended any, the
 // whole CTA inserts the buffered rows into the global table together, Ev::FLUSH_ROWS rows per
 // thread at a time whose first probes are all in flight before the first is waited for, so the global probes and
 // atomics of the cold keys run with all lanes active and overlap.  (A row finding the buffer full goes to the
@@ -1072,7 +1089,7 @@ WS_DI void insertAll(const Launch& L, const Ev& ev, int n, Key&& key, Insert&& i
 // after another (eight queries of up to 2.5M rows into 100 groups: 172 -> 149 us).  A key's copies are used by the rows that see its number; the rows
 // before that went to its slot, and both are merged.
 // Shared memory: [S] key words | [n64][E] accumulators, E = S + kHotKeys * kHotCopies | multi-key [S][nk] key values | [B][rw]
-// buffer | multi-key [B][nk] key values | [n32][E] 32-bit counts | [S] key numbers (bytes, 255: none).
+// buffer | multi-key [B][nk] key values | [n32][E] 32-bit words | [S] key numbers (bytes, 255: none).
 constexpr int kHotKeys = 16, kHotCopies = 8;
 template <class Ev>
 __device__ void aggHash(const Launch& L) {
@@ -1083,7 +1100,7 @@ __device__ void aggHash(const Launch& L) {
   const int S = L.smemSlots, B = L.spillRows;
   const bool multi = nk > 1;
   int n64, n32;
-  compactWords(ev, n64, n32);
+  compactWords(ev, true, n64, n32);
   u64* tkey = wsSmem;
   u64* t64 = tkey + S;
   const int E = S ? S + kHotKeys * kHotCopies : 0;
@@ -1094,7 +1111,7 @@ __device__ void aggHash(const Launch& L) {
   unsigned char* number = (unsigned char*)(t32 + (size_t)E * n32);
   for (int e = threadIdx.x; e < E; e += blockDim.x) {
     if (e < S) tkey[e] = kEmpty, number[e] = 255;
-    compactIdentity(ev, t64, t32, e, E);
+    compactIdentity(ev, true, t64, t32, e, E);
   }
   if (threadIdx.x == 0) spillN = 0, keysN = 0;
   __syncthreads();
@@ -1105,7 +1122,7 @@ __device__ void aggHash(const Launch& L) {
     const u64 kw = keyWord(ev, i, kv);
     u64 x[kMaxRowWords];
     rowOfInput(ev, i, x);
-    if (kw != kEmpty && S > 0 && compactOk(L, ev, x, i)) {
+    if (kw != kEmpty && S > 0) {
       unsigned s = (unsigned)(mix64(kw) & (u64)(S - 1));
 #pragma unroll 1
       for (int p = 0; p < 8; ++p) {
@@ -1123,7 +1140,7 @@ __device__ void aggHash(const Launch& L) {
         if (prev == kw) {
           const unsigned num = *(volatile unsigned char*)(number + s);
           const unsigned e = num < kHotKeys ? S + num * kHotCopies + (lane & (kHotCopies - 1)) : s;
-          compactAdd(ev, x, t64, t32, e, E);
+          compactAdd(ev, true, x, t64, t32, e, E);
           return;
         }
         s = (s + 1) & (S - 1);
@@ -1181,9 +1198,9 @@ __device__ void aggHash(const Launch& L) {
           for (int k = 0; k < nk; ++k) kv[k] = skv[(size_t)s * nk + k];
         u64 w[kMaxRowWords];
         rowIdentity(ev, w);
-        compactInto(ev, w, t64, t32, s, E);
+        compactInto(ev, true, w, t64, t32, s, E);
         if (number[s] < kHotKeys)
-          for (int c = 0; c < kHotCopies; ++c) compactInto(ev, w, t64, t32, S + number[s] * kHotCopies + c, E);
+          for (int c = 0; c < kHotCopies; ++c) compactInto(ev, true, w, t64, t32, S + number[s] * kHotCopies + c, E);
         globalInsert(L, ev, kw, kv, w, first);
       });
 }
@@ -1269,7 +1286,9 @@ __device__ void selectMask(const Launch& L) {
   WS_K_ENTRY_B(PREFIX, nokeys, (ws::aggNoKeys<EV, false>), ws::kThreads, EV::NOKEYS_MIN_BLOCKS)
 #define WS_K_NOKEYS_STAGED(EV, PREFIX) WS_K_ENTRY(PREFIX, nokeys_staged, (ws::aggNoKeys<EV, true>))
 #define WS_K_DENSE_SHARED(EV, PREFIX) \
-  WS_K_ENTRY_B(PREFIX, dense_shared, ws::aggDenseShared<EV>, (ws::kThreads * EV::DENSE_V), 1)
+  WS_K_ENTRY_B(PREFIX, dense_shared, (ws::aggDenseShared<EV, false>), (ws::kThreads * EV::DENSE_V), 1)
+#define WS_K_DENSE_TOPS(EV, PREFIX) \
+  WS_K_ENTRY_B(PREFIX, dense_tops, (ws::aggDenseShared<EV, true>), (ws::kThreads * EV::DENSE_V), 1)
 #define WS_K_DENSE_GLOBAL(EV, PREFIX) WS_K_ENTRY(PREFIX, dense_global, ws::aggDenseGlobal<EV>)
 // The direct-load private-row kernel asks for EV::PRIV_MIN_BLOCKS resident CTAs of kThreads (a
 // register budget); the staged one keeps the producer warp.

@@ -585,11 +585,14 @@ static size_t hashTableBudget(const ws_aggregator& A, bool compact) {
 
 // Bytes of a group's compact accumulators (ws_kern.cuh), and of the hash scan's shared table of `slots` slots: key word,
 // accumulators (also the hot keys' copies), key number, key values of several keys.
-// compact: compiled plans; the interpreter keeps accumulator rows.
-static size_t compactBytes(const ws_aggregator& A, bool compact) {
+// compact: compiled plans; the interpreter keeps accumulator rows.  tops: integer sums have their top words.
+static size_t compactBytes(const ws_aggregator& A, bool compact, bool tops = true) {
   size_t b = 0;
   if (!compact) return (size_t)A.lay.rw * 8;
-  for (int a = 0; a < A.lay.na; ++a) b += A.lay.kind[a] == SK_COUNT ? 4 : A.lay.kind[a] != SK_NONE ? 8 : 0;
+  for (int a = 0; a < A.lay.na; ++a) {
+    const int k = A.lay.kind[a];
+    b += k == SK_COUNT ? 4 : k == SK_ISUM && tops ? 12 : k != SK_NONE ? 8 : 0;
+  }
   return b;
 }
 static size_t hashTableBytes(const ws_aggregator& A, size_t slots, bool compact) {
@@ -713,14 +716,18 @@ static void aggRun(ws_aggregator& A, const ws_expr_env& env, const ws_jit_progra
     const int naEv = ks.interp ? WS_INTERP_AGGS : A.plan.naggs;
     const size_t privBytes = (size_t)G * A.lay.frw * kThreads * 8 + (size_t)G * naEv * 16;
     // compact accumulators per group (ws_kern.cuh), in copies while they are small: few groups meet in a warp
-    const size_t groupBytes = compactBytes(A, !ks.interp);
+    size_t groupBytes = compactBytes(A, !ks.interp);
     int copies = 1;
-    while (!ks.interp && copies < 8 && (size_t)G * copies * 2 * groupBytes <= 24 * 1024) copies <<= 1;
-    const size_t sharedSmem = (size_t)G * copies * groupBytes;
     // A table an SM holds once pays when the CTA brings the SM's warps with it (denseV: 5000 groups of 24 B, 12M rows:
     // 83 us against 377 us of L2 atomics), and where the rows well outnumber the groups each CTA merges
     const int denseV = ks.denseV;
     const size_t sharedLimit = denseV > 1 ? 200 * 1024 : 96 * 1024;
+    // Sums without top words where only they fit: rows of large arguments then go to the global rows, which take them
+    // all otherwise.
+    const bool tops = (size_t)G * groupBytes <= sharedLimit;
+    if (!tops) groupBytes = compactBytes(A, !ks.interp, false);
+    while (!ks.interp && copies < 8 && (size_t)G * copies * 2 * groupBytes <= 24 * 1024) copies <<= 1;
+    const size_t sharedSmem = (size_t)G * copies * groupBytes;
     const bool sharedPays = sharedSmem <= 48 * 1024 || d.rows >= 16 * G;
     if (G * A.lay.frw <= 48 && ks.fn[K_DENSE_PRIV]) {
       // tile stages fit beside the private rows within 220 KB; the staged body is its own entry
@@ -742,7 +749,7 @@ static void aggRun(ws_aggregator& A, const ws_expr_env& env, const ws_jit_progra
           if (st <= fitStages && st != (std::min(maxStages, fitStages) >= 2 ? std::min(maxStages, fitStages) : 0))
             cands.push_back(staged(st));
     } else if (sharedSmem <= sharedLimit && sharedPays && ks.fn[K_DENSE_SHARED]) {
-      CUfunction f = ks.fn[K_DENSE_SHARED];
+      CUfunction f = ks.fn[tops && ks.fn[K_DENSE_TOPS] ? K_DENSE_TOPS : K_DENSE_SHARED];
       L.copies = copies;
       tilesPerCta = denseV;
       shapeOf = [=](const TuneChoice&) { return Shape{f, sharedSmem, kThreads * denseV}; };
