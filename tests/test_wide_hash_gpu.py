@@ -87,6 +87,18 @@ def seconds(e, aq, prog, cap, bufs, n):
     return best, over
 
 
+@pytest.mark.parametrize("jit,narrow,wide", [(True, 8, 22), (False, 2, 6)])
+def test_wide_plans_aggregate_on_chip(jit, narrow, wide):
+    """Few groups: without a shared-memory table a plan of twice the aggregates takes 20 times as long."""
+    n = 4_000_000
+    bufs = [ops.DeviceBuffer.from_array(c) for c in columns(n, 16, 2)]
+    t = {}
+    for aggregates in (narrow, wide):
+        e, aq = query(aggregates, 2)
+        t[aggregates] = seconds(e, aq, program(e, aq, jit), 1024, bufs, n)[0]
+    assert t[wide] < 6 * t[narrow], t
+
+
 @pytest.mark.parametrize("jit", [True, False])
 def test_a_small_table_overflows_early(jit):
     """A run into a table too small for its groups ends soon after the table is 70 % full (the caller reruns with a larger

@@ -27,7 +27,7 @@ SOURCES = ["ws_interp_priv.cu", "ws_interp_hash.cu", "ws_interp_agg.cu", "ws_int
 EMBED = [("kWsTypesSrc", os.path.join(INCLUDE, "ws_types.h")),
          ("kWsDevSrc", os.path.join(CSRC, "ws_dev.cuh")),
          ("kWsKernSrc", os.path.join(CSRC, "ws_kern.cuh"))]
-HEADERS = [p for _, p in EMBED] + [os.path.join(CSRC, f) for f in ("ws_internal.h", "ws_interp.cuh")] + \
+HEADERS = [p for _, p in EMBED] + [os.path.join(CSRC, f) for f in ("ws_internal.h", "ws_interp.cuh", "ws_shape.h")] + \
     [os.path.join(INCLUDE, "ws_b200.h")]
 
 

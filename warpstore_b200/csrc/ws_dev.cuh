@@ -713,7 +713,7 @@ struct Launch {
   int stages;                 // shared-memory stages of staged scans (0: loads straight from global memory)
   int sumShift;               // integer SUM words need no overflow test while (argument magnitude >> sumShift)
                               // is 0 (set at launch from the rows a thread adds; -1: always test)
-  int copies;                 // dense GROUP BY in shared memory: copies of each group (a power of two)
+  int copies;                 // GROUP BY in shared memory: copies of each group (dense) / of the first keys (hash)
   int kmin32;                 // dense GROUP BY: every |kmin| <= 2^30 (32-bit key arithmetic is exact, see denseIndex)
   int waitLog2;               // staged scans: a wait for a tile stage gives up after 2^waitLog2 SM cycles
   // A launch serving several queries gives each its own range of CTAs: this query's first CTA and its

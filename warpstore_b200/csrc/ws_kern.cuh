@@ -969,7 +969,7 @@ __device__ void aggDenseGlobal(const Launch& L) {
       L.err[0] = 1;
       return;
     }
-    u64 x[kMaxRowWords];
+    u64 x[Ev::RW];
     rowOfInput(ev, i, x);
     rowAtomicCombine(ev, L.rows + gi * rw, x);
   });
@@ -1074,21 +1074,23 @@ WS_DI void insertAll(const Launch& L, const Ev& ev, int n, Key&& key, Insert&& i
 }
 
 // Rows are pre-aggregated in a per-CTA shared-memory table (smemSlots key words with compact accumulators,
-// bounded probing), which absorbs hot keys.  A row that finds no slot there is appended to a per-CTA shared buffer (one shared atomic per warp); after a tile that appended any, the
-// whole CTA inserts the buffered rows into the global table together, Ev::FLUSH_ROWS rows per
-// thread at a time whose first probes are all in flight before the first is waited for, so the global probes and
-// atomics of the cold keys run with all lanes active and overlap.  (A row finding the buffer full goes to the
-// global table directly.)  The shared table is merged into the global table when the CTA finishes.
+// bounded probing), which absorbs hot keys.  A row that finds no slot there is appended to a per-CTA shared buffer (one
+// shared atomic per warp); after a tile that appended any, the whole CTA inserts the buffered rows into the
+// global table together, Ev::FLUSH_ROWS rows per thread at a time whose first probes are all in flight before the first
+// is waited for, so the global probes of the cold keys run with all lanes active and overlap.  (A row finding the
+// buffer full goes to the global table directly.)  Every tile ends with a flush, and the shared table is merged into
+// the global table when the CTA finishes.
 // A tile without such rows costs one CTA barrier, which also votes on the flush: a thread knows whether it appended
 // itself, so nobody reads the shared count while others append to it.  (Reading the
 // overflow flag from global memory and three barriers after every tile, with accumulator rows of 64-bit atomics:
 // 1M rows into 16 groups 33.0 -> 24.8 us, 100M Zipf rows into 3.8M groups 4.56 -> 3.26 ms.  The latter is bound by the
 // global table: about one random DRAM sector and three L2 operations per row that is not caught on chip.)
-// The first kHotKeys keys of a CTA also have kHotCopies copies of their accumulators, a lane's copy by its number:
-// with few groups most lanes of a warp meet in a few slots, and their shared atomics on one address run one
-// after another (eight queries of up to 2.5M rows into 100 groups: 172 -> 149 us).  A key's copies are used by the rows that see its number; the rows
-// before that went to its slot, and both are merged.
-// Shared memory: [S] key words | [n64][E] accumulators, E = S + kHotKeys * kHotCopies | multi-key [S][nk] key values | [B][rw]
+// The first kHotKeys keys of a CTA also have L.copies (1: none; up to kHotCopies, as memory allows) copies of their
+// accumulators, a lane's copy by its number: with few groups most lanes of a warp meet in a few slots, and their shared
+// atomics on one address run one after another (eight queries of up to 2.5M rows into 100 groups: 172 -> 149 us).  A key's
+// copies are used by the rows that see its number; the rows before that went to its slot, and both are merged.
+// Sizes of the table, the copies and the buffer: hashTable (ws_shape.h).
+// Shared memory: [S] key words | [n64][E] accumulators, E = S + kHotKeys * copies | multi-key [S][nk] key values | [B][rw]
 // buffer | multi-key [B][nk] key values | [n32][E] 32-bit words | [S] key numbers (bytes, 255: none).
 constexpr int kHotKeys = 16, kHotCopies = 8;
 template <class Ev>
@@ -1103,7 +1105,7 @@ __device__ void aggHash(const Launch& L) {
   compactWords(ev, true, n64, n32);
   u64* tkey = wsSmem;
   u64* t64 = tkey + S;
-  const int E = S ? S + kHotKeys * kHotCopies : 0;
+  const int copies = L.copies, E = S + (copies > 1 ? kHotKeys * copies : 0);
   double* skv = (double*)(t64 + (size_t)E * n64);
   u64* buf = (u64*)skv + (multi ? (size_t)S * nk : 0);
   double* bkv = (double*)(buf + (size_t)B * rw);
@@ -1117,13 +1119,19 @@ __device__ void aggHash(const Launch& L) {
   __syncthreads();
   const int lane = threadIdx.x & 31;
   bool appended = false;  // this thread sent a row to the buffer since the last flush
+  // Interpreter: tiles that go past the shared table.  Its slot loops run for the rows that the table took and again for
+  // the others; where over a quarter of a tile's rows found no slot, the next kSkipTiles tiles only run the second loop
+  // (8M rows, COUNT and eight SUMs into 500 groups: 44 ms with every tile through the table, 19 ms so).
+  constexpr int kSkipTiles = 16;
+  int skip = 0;
   auto rowFn = [&](int i, int, i64) {
     double kv[Ev::NK];
     const u64 kw = keyWord(ev, i, kv);
-    u64 x[kMaxRowWords];
+    u64 x[Ev::RW];
     rowOfInput(ev, i, x);
-    if (kw != kEmpty && S > 0) {
+    if (kw != kEmpty && S > 0 && (Ev::COMPACT || skip == 0)) {
       unsigned s = (unsigned)(mix64(kw) & (u64)(S - 1));
+      bool hit = false;
 #pragma unroll 1
       for (int p = 0; p < 8; ++p) {
         u64 prev = *(volatile u64*)(tkey + s);
@@ -1132,18 +1140,22 @@ __device__ void aggHash(const Launch& L) {
           if (prev == kEmpty) {
             if (multi)
               for (int k = 0; k < nk; ++k) skv[(size_t)s * nk + k] = kv[k];
-            const int num = *(volatile int*)&keysN < kHotKeys ? atomicAdd(&keysN, 1) : kHotKeys;
+            const int num = copies > 1 && *(volatile int*)&keysN < kHotKeys ? atomicAdd(&keysN, 1) : kHotKeys;
             if (num < kHotKeys) *(volatile unsigned char*)(number + s) = (unsigned char)num;
             prev = kw;
           }
         }
         if (prev == kw) {
-          const unsigned num = *(volatile unsigned char*)(number + s);
-          const unsigned e = num < kHotKeys ? S + num * kHotCopies + (lane & (kHotCopies - 1)) : s;
-          compactAdd(ev, true, x, t64, t32, e, E);
-          return;
+          hit = true;
+          break;
         }
         s = (s + 1) & (S - 1);
+      }
+      if (hit) {  // behind the probes, where the lanes that found a slot are together again
+        const unsigned num = *(volatile unsigned char*)(number + s);
+        const unsigned e = num < kHotKeys ? S + num * copies + (lane & (copies - 1)) : s;
+        compactAdd(ev, true, x, t64, t32, e, E);
+        return;
       }
     }
     // bound for the global table: reserve a buffer entry (one shared atomic per warp)
@@ -1169,7 +1181,8 @@ __device__ void aggHash(const Launch& L) {
   auto flush = [&]() -> bool {
     if (!__syncthreads_or(appended)) return false;
     // every thread is past its appends and none appends before the last barrier below
-    const int n = min(spillN, B);
+    const int missed = spillN, n = min(missed, B);
+    if constexpr (!Ev::COMPACT) skip = skip > 0 ? skip - 1 : missed > kTile / 4 ? kSkipTiles : 0;
     if (threadIdx.x == 0) stopFlag = *(volatile int*)(L.err + 1);
     __syncthreads();
     if (threadIdx.x == 0) spillN = 0;
@@ -1196,11 +1209,11 @@ __device__ void aggHash(const Launch& L) {
         double kv[WS_MAX_KEYS];
         if (multi)
           for (int k = 0; k < nk; ++k) kv[k] = skv[(size_t)s * nk + k];
-        u64 w[kMaxRowWords];
+        u64 w[Ev::RW];
         rowIdentity(ev, w);
         compactInto(ev, true, w, t64, t32, s, E);
         if (number[s] < kHotKeys)
-          for (int c = 0; c < kHotCopies; ++c) compactInto(ev, true, w, t64, t32, S + number[s] * kHotCopies + c, E);
+          for (int c = 0; c < copies; ++c) compactInto(ev, true, w, t64, t32, S + number[s] * copies + c, E);
         globalInsert(L, ev, kw, kv, w, first);
       });
 }
@@ -1275,10 +1288,10 @@ __device__ void selectMask(const Launch& L) {
   WS_K_MULTI_B(PREFIX, nokeys, (ws::aggNoKeys<EV, false>), ws::kThreads, EV::NOKEYS_MIN_BLOCKS)
 #define WS_K_MULTI_DENSE_PRIV(EV, PREFIX) \
   WS_K_MULTI_B(PREFIX, dense_priv, (ws::aggDensePriv<EV, false>), ws::kThreads, EV::PRIV_MIN_BLOCKS)
-// The hash scan launches kThreads.  For generated plans EV::HASH_MULTI_MIN_BLOCKS = 3 resident CTAs
-// (the shared table allows them) bound the registers: reading the launch descriptor from shared
-// memory took the kernel from 72 to 82 registers, two CTAs per SM and 20 % more time than the
-// single-query scan; bounded it needs 80, without spills.
+// The hash scan launches kThreads.  For generated plans EV::HASH_MULTI_MIN_BLOCKS resident CTAs (three, two of wide
+// plans: hashMinBlocks) bound the registers: reading the launch descriptor from shared memory takes more of them than
+// the single-query scan does, and unbounded it ran two CTAs per SM and 20 % longer; bounded to 80 registers five
+// aggregates need no spills, seven SUMs 48 bytes.
 #define WS_K_MULTI_HASH(EV, PREFIX) \
   WS_K_MULTI_B(PREFIX, hash, ws::aggHash<EV>, ws::kThreads, EV::HASH_MULTI_MIN_BLOCKS)
 // Direct loads: EV::NOKEYS_MIN_BLOCKS resident CTAs of kThreads; the staged entry keeps the producer warp.

@@ -4,6 +4,7 @@
 #include <cstring>
 
 #include "ws_internal.h"
+#include "ws_shape.h"
 
 namespace ws {
 
@@ -562,48 +563,31 @@ static void aggInitRows(ws_aggregator& A) {
 static TuneChoice tuneScan(ws_aggregator& A, const std::string& key, const std::vector<TuneChoice>& cands,
                            const std::function<void(const TuneChoice&)>& launch);
 
-// Shared-memory budget of the hash scan's per-CTA table in bytes (WARPSTORE_B200_HASH_SMEM_KB overrides).  Where a
-// table of half the global table's capacity (capacities are chosen at twice the expected groups) fits 52 KB the CTA
-// keeps about every group on chip; a table of the whole capacity only costs (eight queries into 100 groups: 178
-// against 149 us).  Beyond that the table catches hot keys and the scan waits for the global table, so resident
-// warps count more than slots: with 24 KB, and as much for the spill buffer, four CTAs fit an SM (100M Zipf rows:
-// 48 + 40 KB and two CTAs 5.39 ms, 24 + 32 KB 3.57 ms, 24 + 24 KB 3.23 ms; 24 + 8 KB overflows into single inserts:
-// 4.90 ms).
-static size_t hashTableBytes(const ws_aggregator& A, size_t slots, bool compact);
-constexpr size_t kHashFitBytes = 52 * 1024, kHashHotBytes = 24 * 1024, kHashSpillBytes = 24 * 1024;
-static size_t hashTableBudget(const ws_aggregator& A, bool compact) {
-  static const int kb = [] {
-    const char* e = getenv("WARPSTORE_B200_HASH_SMEM_KB");
-    const int v = e ? atoi(e) : 0;
-    return v >= 4 && v <= 160 ? v : 0;
-  }();
-  if (kb) return (size_t)kb * 1024;
-  const int64_t s = std::max<int64_t>(A.cap / 2, 64);
-  if (s <= 4096 && hashTableBytes(A, (size_t)s, compact) <= kHashFitBytes) return hashTableBytes(A, (size_t)s, compact);
-  return kHashHotBytes;
-}
-
-// Bytes of a group's compact accumulators (ws_kern.cuh), and of the hash scan's shared table of `slots` slots: key word,
-// accumulators (also the hot keys' copies), key number, key values of several keys.
-// compact: compiled plans; the interpreter keeps accumulator rows.  tops: integer sums have their top words.
-static size_t compactBytes(const ws_aggregator& A, bool compact, bool tops = true) {
-  size_t b = 0;
+// Bytes of a group's accumulators in a shared-memory table (compact words, ws_kern.cuh; the interpreter keeps
+// accumulator rows), integer sums with top words or without.
+static size_t groupBytes(const ws_aggregator& A, bool compact, bool tops = true) {
   if (!compact) return (size_t)A.lay.rw * 8;
+  size_t b = 0;
   for (int a = 0; a < A.lay.na; ++a) {
     const int k = A.lay.kind[a];
     b += k == SK_COUNT ? 4 : k == SK_ISUM && tops ? 12 : k != SK_NONE ? 8 : 0;
   }
   return b;
 }
-static size_t hashTableBytes(const ws_aggregator& A, size_t slots, bool compact) {
-  if (!slots) return 0;
-  return slots * (9 + compactBytes(A, compact) + (A.plan.nkeys > 1 ? (size_t)A.plan.nkeys * 8 : 0)) +
-         kHotKeys * kHotCopies * compactBytes(A, compact);
-}
-static size_t hashSmemSlots(const ws_aggregator& A, size_t budget, bool compact) {
-  size_t s = 4096;
-  while (s > 64 && hashTableBytes(A, s, compact) > budget) s >>= 1;
-  return hashTableBytes(A, s, compact) > budget ? 0 : s;
+
+// The hash scan's shared memory (ws_shape.h); f: its kernel; tableKB: the table's size where tuned or given
+// (WARPSTORE_B200_HASH_SMEM_KB), 0: chosen.
+static HashTable hashTableOf(const ws_aggregator& A, bool compiled, CUfunction f, int tableKB) {
+  static const int envKB = [] {
+    const char* e = getenv("WARPSTORE_B200_HASH_SMEM_KB");
+    const int v = e ? atoi(e) : 0;
+    return v >= 4 && v <= 160 ? v : 0;
+  }();
+  int resident = 0;
+  WS_CKD(drv().occupancy(&resident, f, kThreads, 0));
+  const size_t acc = groupBytes(A, compiled), keys = A.plan.nkeys > 1 ? (size_t)A.plan.nkeys * 8 : 0;
+  return hashTable(A.cap, 9 + keys + acc, acc, kHotKeys, kHotCopies, resident, (size_t)(tableKB > 0 ? tableKB : envKB),
+                   compiled);
 }
 
 // A scan prepared for launching elsewhere (a captured graph): kernel, shape, launch descriptor and the
@@ -716,7 +700,7 @@ static void aggRun(ws_aggregator& A, const ws_expr_env& env, const ws_jit_progra
     const int naEv = ks.interp ? WS_INTERP_AGGS : A.plan.naggs;
     const size_t privBytes = (size_t)G * A.lay.frw * kThreads * 8 + (size_t)G * naEv * 16;
     // compact accumulators per group (ws_kern.cuh), in copies while they are small: few groups meet in a warp
-    size_t groupBytes = compactBytes(A, !ks.interp);
+    size_t perGroup = groupBytes(A, !ks.interp);
     int copies = 1;
     // A table an SM holds once pays when the CTA brings the SM's warps with it (denseV: 5000 groups of 24 B, 12M rows:
     // 83 us against 377 us of L2 atomics), and where the rows well outnumber the groups each CTA merges
@@ -724,10 +708,10 @@ static void aggRun(ws_aggregator& A, const ws_expr_env& env, const ws_jit_progra
     const size_t sharedLimit = denseV > 1 ? 200 * 1024 : 96 * 1024;
     // Sums without top words where only they fit: rows of large arguments then go to the global rows, which take them
     // all otherwise.
-    const bool tops = (size_t)G * groupBytes <= sharedLimit;
-    if (!tops) groupBytes = compactBytes(A, !ks.interp, false);
-    while (!ks.interp && copies < 8 && (size_t)G * copies * 2 * groupBytes <= 24 * 1024) copies <<= 1;
-    const size_t sharedSmem = (size_t)G * copies * groupBytes;
+    const bool tops = (size_t)G * perGroup <= sharedLimit;
+    if (!tops) perGroup = groupBytes(A, !ks.interp, false);
+    while (!ks.interp && copies < 8 && (size_t)G * copies * 2 * perGroup <= 24 * 1024) copies <<= 1;
+    const size_t sharedSmem = (size_t)G * copies * perGroup;
     const bool sharedPays = sharedSmem <= 48 * 1024 || d.rows >= 16 * G;
     if (G * A.lay.frw <= 48 && ks.fn[K_DENSE_PRIV]) {
       // tile stages fit beside the private rows within 220 KB; the staged body is its own entry
@@ -773,14 +757,14 @@ static void aggRun(ws_aggregator& A, const ws_expr_env& env, const ws_jit_progra
     L.count = A.count();
     L.probeLimit = (int)std::min<int64_t>(A.cap, 1 << 16);
     const size_t per = (size_t)A.lay.rw * 8 + (A.plan.nkeys > 1 ? (size_t)A.plan.nkeys * 8 : 0);
-    L.spillRows = (int)std::min<size_t>(kTile, kHashSpillBytes / per);
     ws_aggregator* ap = &A;
-    const bool compact = !ks.interp;
+    const bool compiledPlan = !ks.interp;
     shapeOf = [=](const TuneChoice& c) {
-      // per-CTA table: up to 4096 slots within the budget
-      const size_t slots = hashSmemSlots(*ap, c.smemKB > 0 ? (size_t)c.smemKB * 1024 : hashTableBudget(*ap, compact), compact);
-      lp->smemSlots = (int)slots;
-      return Shape{f, hashTableBytes(*ap, slots, compact) + (size_t)lp->spillRows * per, kThreads};
+      const HashTable t = hashTableOf(*ap, compiledPlan, f, c.smemKB);
+      lp->smemSlots = (int)t.slots;
+      lp->copies = t.copies;
+      lp->spillRows = (int)std::min<size_t>(kTile, t.spill / per);
+      return Shape{f, t.bytes + (size_t)lp->spillRows * per, kThreads};
     };
     name = "hash";
     for (int kb : {16, 32, 96}) {
