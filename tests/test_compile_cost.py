@@ -1,9 +1,12 @@
 """What a new query shape compiles (no GPU: NVRTC targets sm_100a): kernels for batches stored otherwise than hinted and staged
-kernels are not part of a plan's module."""
+kernels are not part of a plan's module, the hash scan holds one copy of its insertion per place, and the register
+bounds follow the plan's width."""
 import os
 import re
 import subprocess
 import sys
+
+import pytest
 
 ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
 CHILD = r"""
@@ -45,3 +48,9 @@ def test_dense_module_has_no_staged_kernels(built):
     _, names = compiled("dense", 4, 1)
     assert names and not any("staged" in n or n.startswith("wsg_") for n in names), names
 
+
+@pytest.mark.parametrize("sums,limit", [(7, 400), (16, 500), (25, 1200)])
+def test_register_bounds_follow_the_width(built, sums, limit):
+    """Spill stores of the single-query hash scan (25 SUMs under the bound of narrow plans: over 5000 bytes)."""
+    _, spills = compiled("hash", sums, 0)
+    assert spills["wsq_hash"] <= limit, spills

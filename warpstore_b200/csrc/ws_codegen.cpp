@@ -272,6 +272,18 @@ const char* valType(const ColUse& u) {
 
 }  // namespace
 
+// Resident CTAs that the hash scan's registers are bounded for, at most `most`: `words` 32-bit words hold a thread's four
+// rows, and an accumulator's argument and addresses take about four registers.  Past the bound the kernel spills;
+// the scan waits for shared and L2 atomics meanwhile, so moderate spills cost less than warps do (8M rows, us under
+// the bounds 4 / 3 / 2; 16 groups: 10 SUMs of two columns (64 by this measure) 203 / 216 / 258, five SUMs of five columns (68)
+// 198 / 158 / 130, 16 SUMs of two columns (88) 691 / 321 / 348, 25 SUMs (124) 1036 / 1439 / 602; 100,000 groups: 1708 / 2958 / 4051, 784 /
+// 1030 / 1600, 2994 / 2688 / 5271; eight SUMs of eight columns (104) into 500 groups 749 / 686 / 1145).
+int hashMinBlocks(int words, const SlotLayout& lay, int most) {
+  int regs = words;
+  for (int a = 0; a < lay.na; ++a) regs += lay.kind[a] != SK_NONE ? 4 : 0;
+  return std::min(most, regs <= 64 ? 4 : regs <= 110 ? 3 : 2);
+}
+
 // Generated evaluator for one plan (see the evaluator contract in ws_kern.cuh).
 std::string genEvaluator(const ws_expr_env& env, int ncols, const ws_agg_plan& plan, int fnKind, int* stageBytesOut) {
   Gen g{env, ncols};
@@ -323,7 +335,10 @@ std::string genEvaluator(const ws_expr_env& env, int ncols, const ws_agg_plan& p
     return v >= 1 && v <= 4 ? v : 2;
   }();
   o << "  static constexpr int PRIV_MIN_BLOCKS = " << privMinBlocks << ";\n";
-  o << "  static constexpr int HASH_MIN_BLOCKS = 3, HASH_MULTI_MIN_BLOCKS = 3;\n";  // the multi-query hash scan's register bound
+  int valueWords = 0;  // of four decoded rows
+  for (auto& [c, u] : g.cols) valueWords += u.vec ? 0 : u.t == 0 || u.t == 3 ? 4 : 8;
+  const int hashBlocks = hashMinBlocks(valueWords, lay, 3);
+  o << "  static constexpr int HASH_MIN_BLOCKS = " << hashBlocks << ", HASH_MULTI_MIN_BLOCKS = " << hashBlocks << ";\n";
   o << "  static constexpr int NOKEYS_MIN_BLOCKS = 1, SELECT_MIN_BLOCKS = 1, DENSE_V = 1, FLUSH_ROWS = 4;\n  static constexpr bool HOT = false, COMPACT = true;\n  static constexpr unsigned KEY32 = 0;\n";
   o << "  static constexpr int NSC = " << std::max<size_t>(staged.size(), 1) << ", STAGE_BYTES = " << stageBytes << ";\n";
   o << "  struct Stage { const unsigned char* d[NSC]; int w[NSC]; unsigned bytes; int ok; };\n";
@@ -499,7 +514,9 @@ std::string genEvaluator(const ws_expr_env& env, int ncols, const ws_agg_plan& p
 
 
 // Groups of kThreads threads in a CTA of the shared-table dense scan (ws_kern.cuh): four, 64 registers a thread,
-// where the fetched words leave room in them, else two.
+// where the fetched words leave room in them, else two.  Accumulators do not count: wide plans spill, and still run
+// faster than with half the warps (8M rows into 40 groups, four / two: 11 SUMs 96 / 126 us, 16 SUMs 139 / 167, 25 SUMs
+// 231 / 247).
 static int hotDenseV(int words) { return words <= 28 ? 4 : 2; }
 
 // Evaluator (struct QHot) of a plan whose columns are stored as their hints say: raw, or every segment in the
@@ -571,7 +588,8 @@ std::string genHot(const ws_expr_env& env, int ncols, const ws_agg_plan& plan, i
   o << "  static constexpr int NK = " << std::max(nk, 1) << ", NA = " << na << ", RW = " << (agg ? lay.rw : 1)
     << ", FRW = " << frw << ";\n";
   o << "  static constexpr bool STAGED = false, HOT = true, COMPACT = true;\n  static constexpr int STAGE_BYTES = 0;\n";
-  o << "  static constexpr int PRIV_MIN_BLOCKS = " << privMinBlocks << ", HASH_MIN_BLOCKS = 4, HASH_MULTI_MIN_BLOCKS = 3, NOKEYS_MIN_BLOCKS = "
+  o << "  static constexpr int PRIV_MIN_BLOCKS = " << privMinBlocks << ", HASH_MIN_BLOCKS = " << hashMinBlocks(words, lay, 4)
+    << ", HASH_MULTI_MIN_BLOCKS = " << hashMinBlocks(words, lay, 3) << ", NOKEYS_MIN_BLOCKS = "
     << minBlocks << ", SELECT_MIN_BLOCKS = 4, DENSE_V = " << hotDenseV(words) << ", FLUSH_ROWS = 4;\n";
   unsigned key32 = 0;
   for (int k = 0; k < nk; ++k)
