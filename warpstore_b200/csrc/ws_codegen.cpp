@@ -47,10 +47,10 @@ int jitMode() { return tMode >= 0 ? tMode : gDefaultMode.load(); }
 struct Sym {
   std::string e;
   bool isInt;
-  // The narrow form of an integer expression (see genHot): its value as an int (kind 1) or an i64 (kind 2) of
-  // magnitude below 2^bits, valid in rows that raise no narrow flag; kind 0: none.
+  // The narrow form of an integer expression (see genHot): its value as an int (kind 1) or, of a product, as an i64
+  // (kind 2), valid in rows that raise no narrow flag; kind 0: none.
   std::string n = "";
-  int kind = 0, bits = 0;
+  int kind = 0;
   int ncol = -1, nconst = -1;  // kind 1: the column / constant that must fit in int32 (checked once a row / thread)
   std::string stmt = "";       // statements computing n into the variable $
 };
@@ -85,7 +85,7 @@ struct Gen {
     Sym t{"t" + j + "[i]", r.isInt};
     std::string stmt;
     if (r.kind && !r.stmt.empty()) {
-      t.kind = r.kind, t.bits = r.bits, t.n = "n" + j;
+      t.kind = r.kind, t.n = "n" + j;
       for (char c : r.stmt) stmt += c == '$' ? t.n : std::string(1, c);
     }
     tempOf.emplace(r.e, t);
@@ -108,18 +108,14 @@ struct Gen {
         x[j] = useNarrow(*k[j]);
         if (k[j]->kind == 2) pre += "w|=ws::wide32(" + x[j] + ");", narrowChecked.insert(x[j]);
       }
-      r.kind = 2, r.bits = 62;
+      r.kind = 2;
       r.stmt = pre + "const ws::i64 $=(ws::i64)(int)(" + x[0] + ")*(ws::i64)(int)(" + x[1] + ");";
     } else if (a.kind == 1 && b.kind == 1) {
       const std::string A = useNarrow(a), B = useNarrow(b), o = op == WS_OP_ADD ? "+" : "-";
-      r.kind = 1, r.bits = 31;
+      r.kind = 1;
       r.stmt = "const int $=(int)((unsigned)(" + A + ")" + o + "(unsigned)(" + B + "));ov|=((" + A + ")^" +
                (op == WS_OP_ADD ? "$" : "(" + B + ")") + ")&(" + (op == WS_OP_ADD ? "(" + B + ")" : "(" + A + ")") + "^$);";
-    } else if (std::max(a.bits, b.bits) < 62) {
-      r.kind = 2, r.bits = std::max(a.bits, b.bits) + 1;
-      r.stmt = "const ws::i64 $=(ws::i64)(" + useNarrow(a) + ")" + (op == WS_OP_ADD ? "+" : "-") + "(ws::i64)(" +
-               useNarrow(b) + ");";
-    }
+    }  // the sum of a product has no narrow form: it may need 64 bits
   }
 
   void useCol(int c, bool vecOnly) {
@@ -153,7 +149,7 @@ struct Gen {
         const std::string v = cv(n.arg);
         if (ty == 0 || ty == 1) {
           Sym r{"((ws::i64)" + v + ")", true};
-          r.n = "(int)" + v, r.kind = 1, r.bits = 31, r.ncol = ty == 1 ? n.arg : -1;
+          r.n = "(int)" + v, r.kind = 1, r.ncol = ty == 1 ? n.arg : -1;
           return r;
         }
         if (ty == 2) return {v, false};
@@ -175,7 +171,7 @@ struct Gen {
         if (n.isInt) {
           iconsts.insert(n.arg);
           Sym r{"ik" + arg + "()", true};
-          r.n = "(int)ik" + arg + "()", r.kind = 1, r.bits = 31, r.nconst = n.arg;
+          r.n = "(int)ik" + arg + "()", r.kind = 1, r.nconst = n.arg;
           return r;
         }
         dconsts.insert(n.arg);

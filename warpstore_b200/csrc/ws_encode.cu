@@ -51,19 +51,16 @@ WS_DI void ctaAtomicMin(u64 m, u64* red, unsigned long long* out) {
   }
 }
 
-// st (all bytes 0xff before): st[0] = ordU(min) of the non-NULL values, st[1] = ~ordU(max), st[2] = 0 when any
-// value is NULL
+// st (all bytes 0xff before): st[0] = ordU(min) of the non-NULL values, st[1] = ~ordU(max)
 __global__ void kMinMax(const void* src, int i32, long long nul, int64_t n, unsigned long long* st) {
   __shared__ u64 red[32];
-  u64 mn = ~0ull, mx = ~0ull, noNull = ~0ull;
+  u64 mn = ~0ull, mx = ~0ull;
   WS_GRID_STRIDE(i, n) {
     const long long v = rawAt(src, i32, i);
-    if (v == nul) noNull = 0;
-    else mn = min(mn, ordU(v)), mx = min(mx, ~ordU(v));
+    if (v != nul) mn = min(mn, ordU(v)), mx = min(mx, ~ordU(v));
   }
   ctaAtomicMin(mn, red, st);
   ctaAtomicMin(mx, red, st + 1);
-  ctaAtomicMin(noNull, red, st + 2);
 }
 
 // Segment header (16 bytes) and the 16 pad bytes after the payload, written by the encoding kernels' first CTA
@@ -368,9 +365,9 @@ int ws_encode_column(const void* src, int t, int64_t n, int enc, void** out, int
     if (n < 0 || n > INT32_MAX) throw Error("encode: segment row count out of range", WS_ERR_ARG);
     const int i32 = t == WS_T_I32 || t == WS_T_I32N;
     const long long nul = i32 ? (long long)WS_NULL_I32 : (long long)WS_NULL_I64;
-    // statistics: min / max / NULL and the run count
-    DBuf<unsigned long long> st(3);
-    WS_CK(cudaMemsetAsync(st.p, 0xff, 8 * 3, stream()));
+    // statistics: min / max and the run count
+    DBuf<unsigned long long> st(2);
+    WS_CK(cudaMemsetAsync(st.p, 0xff, 8 * 2, stream()));
     if (n) WS_LAUNCH(kMinMax, gridFor(n, 256, 4), 256, 0, src, i32, nul, n, st.p);
     const int64_t nchunks = std::max<int64_t>((n + 1023) / 1024, 1);
     DBuf<int64_t> counts(nchunks + 1);
@@ -380,7 +377,7 @@ int ws_encode_column(const void* src, int t, int64_t n, int enc, void** out, int
     } else {
       WS_CK(cudaMemsetAsync(counts.p, 0, 8 * (nchunks + 1), stream()));
     }
-    unsigned long long hs[3];
+    unsigned long long hs[2];
     int64_t runs = 0;
     WS_CK(cudaMemcpyAsync(hs, st.p, sizeof hs, cudaMemcpyDeviceToHost, stream()));
     WS_CK(cudaMemcpyAsync(&runs, counts.p + nchunks, 8, cudaMemcpyDeviceToHost, stream()));
@@ -433,10 +430,10 @@ int ws_encode_column_engine(const void* src, int ptype, int64_t n, void** out, i
     if (ptype != WS_PT_F64) {  // frame of reference
       const int i32 = ptype == WS_PT_I32;
       const long long nul = i32 ? (long long)WS_NULL_I32 : (long long)WS_NULL_I64;
-      DBuf<unsigned long long> st(3);
-      WS_CK(cudaMemsetAsync(st.p, 0xff, 8 * 3, stream()));
+      DBuf<unsigned long long> st(2);
+      WS_CK(cudaMemsetAsync(st.p, 0xff, 8 * 2, stream()));
       WS_LAUNCH(kMinMax, gridFor(n, 256, 4), 256, 0, src, i32, nul, n, st.p);
-      unsigned long long hs[3];
+      unsigned long long hs[2];
       d2hSync(hs, st.p, sizeof hs);
       long long mn = unordU(hs[0]), mx = unordU(~hs[1]);
       if (mn > mx) mn = mx = 0;  // every value NULL
