@@ -7,17 +7,8 @@
 
 namespace ws {
 
-// Stored integer of any integer view (raw or encoded), the type's NULL sentinel for NULL.
-WS_DI i64 colIntAt(const ws_col_view& v, i64 r) {
-  const bool i32 = v.t == 0 || v.t == 3;
-  if (!v.enc) return i32 ? (i64)__ldg((const int*)v.p + r) : __ldg((const i64*)v.p + r);
-  const i64 nul = i32 ? (i64)WS_NULL_I32 : (i64)WS_NULL_I64;
-  if (v.enc >= 7) {
-    i64 o[4];
-    load4encView(o, &v, r, nul, 1);
-    return o[0];
-  }
-  const ColRef c = resolveCol(v);
+// Row r of a resolved column: the integer of encodings 1-3 (nul for NULL), the double of encodings 4-6 (NaN for NULL).
+WS_DI i64 encIntAt(const ColRef& c, i64 r, i64 nul) {
   unsigned code;
   if (c.enc == 1) {
     code = __ldg(c.d + r);
@@ -30,13 +21,26 @@ WS_DI i64 colIntAt(const ws_col_view& v, i64 r) {
   code = __ldg((const unsigned*)c.d + r);
   return code == 0xffffffffu ? nul : c.base + (i64)code;
 }
-WS_DI double colDblAt(const ws_col_view& v, i64 r) {
-  if (!v.enc) return __ldg((const double*)v.p + r);
-  const ColRef c = resolveCol(v);
+WS_DI double encDblAt(const ColRef& c, i64 r) {
   if (c.enc == 4) return __ldg(c.dict + __ldg(c.d + r));
   const unsigned code = c.enc == 5 ? (unsigned)__ldg((const unsigned short*)c.d + r) : __ldg((const unsigned*)c.d + r);
   const unsigned nulc = c.enc == 5 ? 0xffffu : 0xffffffffu;
   return code == nulc ? nanv() : (double)(c.base + (i64)code) / c.p10;
+}
+// Stored integer of any integer view (raw or encoded), the type's NULL sentinel for NULL.
+WS_DI i64 colIntAt(const ws_col_view& v, i64 r) {
+  const bool i32 = v.t == 0 || v.t == 3;
+  if (!v.enc) return i32 ? (i64)__ldg((const int*)v.p + r) : __ldg((const i64*)v.p + r);
+  const i64 nul = i32 ? (i64)WS_NULL_I32 : (i64)WS_NULL_I64;
+  if (v.enc >= 7) {
+    i64 o[4];
+    load4encView(o, &v, r, nul, 1);
+    return o[0];
+  }
+  return encIntAt(resolveCol(v), r, nul);
+}
+WS_DI double colDblAt(const ws_col_view& v, i64 r) {
+  return v.enc ? encDblAt(resolveCol(v), r) : __ldg((const double*)v.p + r);
 }
 WS_DI double pow10d(int s) {
   double p = 1;

@@ -130,22 +130,16 @@ WS_DI void gatherBatch(GatherBatch& g, const ws_col_view* src, const int64_t* bo
   g.v = src[lo];
   g.lo = boff[lo];
   g.hi = lo + 1 < nb ? boff[lo + 1] : INT64_MAX;
-  if (g.v.enc && g.v.enc < 7) g.c = resolveCol(g.v);
+  if (g.v.enc) g.c = resolveCol(g.v);
 }
 template <class T>  // int32_t, int64_t or double: the raw storage of ptype
 WS_DI T gatherOne(const GatherBatch& g, int64_t r) {
   if (!g.v.enc) return __ldg((const T*)g.v.p + r);
   if constexpr (sizeof(T) == 8 && T(0.5) != T(0)) {  // double
-    if (g.c.enc == 4) return __ldg(g.c.dict + __ldg(g.c.d + r));
-    const unsigned code = g.c.enc == 5 ? (unsigned)__ldg((const unsigned short*)g.c.d + r) : __ldg((const unsigned*)g.c.d + r);
-    return code == (g.c.enc == 5 ? 0xffffu : 0xffffffffu) ? nanv() : (double)(g.c.base + (i64)code) / g.c.p10;
+    return encDblAt(g.c, r);
   } else {
     if (g.v.enc >= 7) return (T)colIntAt(g.v, r);
-    const i64 nul = sizeof(T) == 4 ? (i64)WS_NULL_I32 : (i64)WS_NULL_I64;
-    const unsigned code = g.c.enc == 1 ? (unsigned)__ldg(g.c.d + r)
-                          : g.c.enc == 2 ? (unsigned)__ldg((const unsigned short*)g.c.d + r) : __ldg((const unsigned*)g.c.d + r);
-    const unsigned top = g.c.enc == 1 ? 0xffu : g.c.enc == 2 ? 0xffffu : 0xffffffffu;
-    return (T)(code == top ? nul : g.c.base + (i64)code);
+    return (T)encIntAt(g.c, r, sizeof(T) == 4 ? (i64)WS_NULL_I32 : (i64)WS_NULL_I64);
   }
 }
 template <class T>
