@@ -1,5 +1,8 @@
-"""Batches stored otherwise than their plan's hints while the kernels for them are compiled in the background (the default
-mode): every run in between and after, a multi-query launch and a prepared query give the oracle's groups."""
+"""Batches stored otherwise than their plan's hints, plans compiled in the background (the default mode): runs, a
+multi-query launch and a prepared query give the oracle's groups, and a process may end as soon as its plan was used."""
+import os
+import subprocess
+import sys
 import time
 
 import numpy as np
@@ -41,7 +44,7 @@ def prepared(kind, stored, seed):
 
 
 @pytest.mark.parametrize("kind", ["hash", "dense"])
-def test_runs_while_the_kernels_compile(kind):
+def test_runs_of_background_plans(kind):
     e, aq, ds, host, dev, keep = prepared(kind, 0, 1)
     fn = abi.JF_DENSE if kind == "dense" else abi.JF_GROUPED
     ok, ow, _ = oracle.aggregate(e.env, aq.plan, host, e.ncols)
@@ -53,7 +56,7 @@ def test_runs_while_the_kernels_compile(kind):
             time.sleep(0.01)
         assert prog
         t0 = time.time()
-        while time.time() - t0 < 8:  # the kernels for other storage become ready meanwhile
+        while time.time() - t0 < 1:
             agg = ops.GpuAggregator(aq.plan, 64, ds)
             agg.add_batches(e.ncols, dev)
             agg.run(e.env, prog)
@@ -80,8 +83,7 @@ def test_runs_while_the_kernels_compile(kind):
         ops.jit_set_mode(-1)
 
 
-def test_a_prepared_query_waits_for_its_kernels():
-    """Created right after its plan, before the kernels for its storage are there."""
+def test_a_prepared_query_of_a_new_plan():
     e, aq, ds, host, dev, keep = prepared("hash", 0, 2)
     aq = q.AggQuery(e, q.col(1).lt(200), [(q.col(0), True)], [q.Agg("COUNT"), q.Agg("MIN", q.col(1), "BIGINT", True)])
     raw = [np.random.default_rng(9).integers(0, 250, n) for n in (4000, 77)]
@@ -108,3 +110,34 @@ def test_a_prepared_query_waits_for_its_kernels():
         ex.close()
     finally:
         ops.jit_set_mode(-1)
+
+
+CHILD = r"""
+import time
+import numpy as np
+from warpstore_b200 import abi, ops
+from warpstore_b200 import query as q
+e = q.Env()
+e.column(abi.T_I32, 0, 0)
+e.column(abi.T_I64, 0, 2)
+aq = q.AggQuery(e, q.col(1).lt(300), [(q.col(0), True)], [q.Agg("COUNT"), q.Agg("SUM", q.col(1), "BIGINT", True)])
+prog = None
+while not prog:
+    prog = ops.jit_get(e.env, e.ncols, aq.plan, abi.JF_GROUPED, "test")
+    time.sleep(0.005)
+k, v = np.arange(5000, dtype=np.int32) % 7, np.arange(5000) % 500
+bufs = [ops.DeviceBuffer.from_array(x) for x in (k, v)]
+agg = ops.GpuAggregator(aq.plan, 64)
+agg.add_batches(e.ncols, [(5000, 0, [abi.ColView(bufs[0].ptr, abi.T_I32, 0, 0, 0), abi.ColView(bufs[1].ptr, abi.T_I64, 0, 0, 0)])])
+agg.run(e.env, prog)
+assert agg.fetch()[0].shape == (7, 1)
+agg.close()
+"""
+
+
+def test_a_process_may_end_after_its_first_run():
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    for _ in range(2):
+        r = subprocess.run([sys.executable, "-c", CHILD], cwd=root, env=dict(os.environ, PYTHONPATH=root), capture_output=True,
+                           text=True, timeout=120)
+        assert r.returncode == 0, r.stderr[-2000:]

@@ -757,8 +757,8 @@ std::string stagedKernels(int fnKind) {
 }
 // A plan's sources.  `evaluators` (QEv, QHot) identify the plan.  With a QHot its direct kernels (prefix wsq) are compiled
 // when the plan is asked for; QEv's run batches stored otherwise than hinted (some hint is an encoding) and
-// are compiled at the first call with such a batch, staged kernels (QEv) at the first staged launch: compiling all of
-// them with the plan took 1.2 to 6 times as long (five aggregates over encoded columns 4.5 -> 19.7 s).  A plan without
+// are compiled behind them in the background, or in WS_JIT_SYNC at the first call with such a batch; staged kernels (QEv)
+// at the first staged launch: compiling all of them in one module took 1.2 to 6 times as long (five aggregates over encoded columns 4.5 -> 19.7 s).  A plan without
 // GROUP BY has its QEv kernels at once: they are small, and the no-allocation entry cannot compile.
 struct PlanSource {
   std::string evaluators, main, any, staged;
@@ -958,12 +958,12 @@ void compileProgram(ws_jit_program& p) {
   }
 }
 
-// Compiles a module of p at its first use, once (state: see ws_jit_program).
+// Compiles a module of p once (state: see ws_jit_program).
 void compileLater(const ws_jit_program& p, const std::string& source, const char* prefix, KernelSet& set,
                   std::atomic<int>& state) {
+  if (state.load(std::memory_order_acquire) != 0) return;
   std::lock_guard<std::mutex> g(p.buildMu);
-  const int st = state.load(std::memory_order_acquire);
-  if (st == 1 || st == 2) return;
+  if (state.load(std::memory_order_acquire) != 0) return;
   bool ok = false;
   try {
     findKernels(compileModule(source, nullptr), prefix, set);
@@ -975,11 +975,14 @@ void compileLater(const ws_jit_program& p, const std::string& source, const char
 }
 void compileAny(const ws_jit_program& p) { compileLater(p, p.anySource, "wsg_", p.any, p.anyState); }
 
-void compileAndPublish(const std::shared_ptr<ws_jit_program>& p) {
+// all: with the kernels for other storage, so that nothing is left to compile in the background once the plan is ready
+// (a process must not end beneath the compiler).
+void compileAndPublish(const std::shared_ptr<ws_jit_program>& p, bool all) {
   auto t0 = std::chrono::steady_clock::now();
   bool ok = false;
   try {
     compileProgram(*p);
+    if (all && !p->anySource.empty()) compileAny(*p);
     ok = true;
   } catch (const std::exception& e) {
     fprintf(stderr, "[warpstore_b200] codegen failed, using the interpreter: %s\n", e.what());
@@ -994,13 +997,8 @@ void compileAndPublish(const std::shared_ptr<ws_jit_program>& p) {
 
 using namespace ws;
 
-const KernelSet* ws_jit_program::anyStorage(bool wait) const {
-  int st = anyState.load(std::memory_order_acquire);
-  if (st == 0 && !wait && !sync && anyState.compare_exchange_strong(st, 3)) {
-    std::shared_ptr<const ws_jit_program> p = shared_from_this();
-    std::thread([p] { compileAny(*p); }).detach();
-  }
-  if (wait || sync) compileAny(*this);
+const KernelSet* ws_jit_program::anyStorage() const {
+  compileAny(*this);
   return anyState.load(std::memory_order_acquire) == 1 ? &any : nullptr;
 }
 CUfunction ws_jit_program::stagedKernel(KernelId k) const {
@@ -1085,20 +1083,16 @@ int ws_jit_get(const ws_expr_env* env, int ncols, const ws_agg_plan* plan, int f
       if (gByShape.size() >= kMaxShapes) gByShape.clear();
       gByShape[shape] = p;
     }
-    if (mode == WS_JIT_SYNC) p->sync = true;
     if (fresh) {
       if (mode == WS_JIT_SYNC) {
-        compileAndPublish(p);
+        compileAndPublish(p, false);
         if (p->state.load() == 1) {
           if (p->fromDisk) ++tInfo.from_disk;
           else ++tInfo.compiled;
           tInfo.compile_ms += p->compileMs;
         }
       } else {
-        std::thread([p] {  // run interpreted now, compiled next time
-          compileAndPublish(p);
-          if (p->state.load() == 1 && !p->anySource.empty()) compileAny(*p);
-        }).detach();
+        std::thread([p] { compileAndPublish(p, true); }).detach();  // run interpreted now, compiled next time
       }
     } else if (mode == WS_JIT_SYNC) {
       for (int spins = 0; p->state.load(std::memory_order_acquire) == 0; ++spins)  // compiled by another thread

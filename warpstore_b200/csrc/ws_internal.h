@@ -175,12 +175,13 @@ unsigned persistentGrid(CUfunction f, size_t smem, int64_t ntiles, int threads =
 
 // A compiled plan (the engine's JitProgram, src/jit.h:16-31): generated evaluator source, its module
 // and kernels, state and statistics.
-struct ws_jit_program : std::enable_shared_from_this<ws_jit_program> {
+struct ws_jit_program {
   int id = 0;
   int fnKind = 0;
   std::string kind, sql, source;
-  // The module compiled when a plan is asked for (every direct-load kernel of its evaluator), and those compiled at the
-  // first call that needs them: kernels for batches stored otherwise than hinted, and staged kernels ("": none).
+  // The module of every direct-load kernel of the plan's evaluator; the one for batches stored otherwise than hinted
+  // (compiled behind it in the background, or at the first such batch of a plan asked for in WS_JIT_SYNC) and the one of
+  // the staged kernels (at the first staged launch); "": none.
   std::string mainSource, anySource, stagedSource;
   // hot: `kernels` are instantiated with the evaluator of hinted storage, which only runs batches whose columns
   // are stored as `encs` (column, encoding) says; `any` runs any batch the plan covers.
@@ -191,20 +192,18 @@ struct ws_jit_program : std::enable_shared_from_this<ws_jit_program> {
   bool fromDisk = false;
   int stageBytes = 0;  // shared memory per staged tile (0: the plan reads global memory directly)
   ws::KernelSet kernels;
-  mutable ws::KernelSet any, staged;                         // filled by anyStorage / stagedKernel
-  mutable std::atomic<int> anyState{0}, stagedState{0};      // 0 not compiled, 1 ready, 2 failed, 3 compiling (another thread)
-  mutable std::mutex buildMu;                                // held while one of them is compiled
-  std::atomic<bool> sync{false};  // asked for in WS_JIT_SYNC: its later modules are waited for too
-  // The kernels that can run these batches; null: not compiled yet, and the caller (wait false) interprets the
-  // plan meanwhile, as it does while the plan itself is compiled.
-  const ws::KernelSet* kernelsFor(int nb, int ncols, const ws_col_view* bcols, bool wait) const {
+  mutable ws::KernelSet any, staged;                     // filled by anyStorage / stagedKernel
+  mutable std::atomic<int> anyState{0}, stagedState{0};  // 0 not compiled, 1 ready, 2 failed
+  mutable std::mutex buildMu;                            // held while one of them is compiled
+  // The kernels that can run these batches; null: they failed to compile (the caller interprets the plan).
+  const ws::KernelSet* kernelsFor(int nb, int ncols, const ws_col_view* bcols) const {
     if (!hot) return &kernels;
     for (int b = 0; b < nb; ++b)
       for (auto& [c, e] : encs)
-        if (bcols[(int64_t)b * ncols + c].enc != e) return anyStorage(wait);
+        if (bcols[(int64_t)b * ncols + c].enc != e) return anyStorage();
     return &kernels;
   }
-  const ws::KernelSet* anyStorage(bool wait) const;
+  const ws::KernelSet* anyStorage() const;
   CUfunction stagedKernel(ws::KernelId k) const;  // compiled when first asked for; null: none
   CUmodule module = nullptr;
   std::mutex mu;

@@ -117,7 +117,7 @@ extern "C" int ws_agg_nokeys_noalloc(const ws_expr_env* env, int ncols, const ws
     }
     ensureInit();
     unsigned char* s = scratchOnDevice();
-    const KernelSet& ks = useJit ? *jit->kernelsFor(nb, ncols, bcols, false) : interpKernels();
+    const KernelSet& ks = useJit ? *jit->kernelsFor(nb, ncols, bcols) : interpKernels();
     CUfunction f = ks.fn[K_NOKEYS];
     unsigned grid = persistentGrid(f, 0, std::max<int64_t>(ntiles, 1));
     const unsigned maxGrid = (unsigned)(kPartBytes / (8 * (size_t)lay.rw));

@@ -614,9 +614,8 @@ static void aggRun(ws_aggregator& A, const ws_expr_env& env, const ws_jit_progra
   if (nb == 0) return;
   A.newRun();
   const bool interpretable = A.plan.naggs <= WS_INTERP_AGGS && A.plan.nkeys <= WS_INTERP_KEYS;
-  // a prepared query keeps the kernel it gets, and a plan the interpreter cannot run has no other: both wait for it
   const KernelSet* compiled = jit && jit->state.load() == 1 && planCovers(env, nb, A.ncols, A.bcols.data())
-                                  ? jit->kernelsFor(nb, A.ncols, A.bcols.data(), prep || !interpretable) : nullptr;
+                                  ? jit->kernelsFor(nb, A.ncols, A.bcols.data()) : nullptr;
   const bool useJit = compiled != nullptr;
   if (!useJit && !interpretable)
     throw Error("this aggregation needs a compiled plan (more than 16 aggregates or 4 GROUP BY keys); codegen failed or is off", WS_ERR_PLAN);

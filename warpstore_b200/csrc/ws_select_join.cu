@@ -761,7 +761,7 @@ static int64_t selectRun(const ws_expr_env& env, bool hasWhere, ws_prog where, i
         if (bcols[(int64_t)b * ncols + c].enc && !env.cols[c].enc) return false;
     return true;
   }();
-  const KernelSet* compiled = covered ? jit->kernelsFor(nb, ncols, bcols, false) : nullptr;
+  const KernelSet* compiled = covered ? jit->kernelsFor(nb, ncols, bcols) : nullptr;
   std::unique_ptr<TProgs> progs;
   if (!compiled) {
     progs.reset(new TProgs);
